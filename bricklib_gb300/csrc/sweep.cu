@@ -1,4 +1,5 @@
 // Host side of the sweep: stencil analysis, kernel selection, bk_sweep and bk_steps.
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <string>
@@ -26,6 +27,122 @@ static int shape_of(const Layout &L) {
   if (L.bk == 16 && L.bj == 8 && L.bi == 8) return 2;
   if (L.bk == 8 && L.bj == 8 && L.bi == 32) return 3;
   return -1;
+}
+
+// The fixed-point form of a stencil (fx.cuh): n taps with coefficients c; near[m] lists (up to 8,
+// terminated by -1) the positions in c of the taps at distance one on the axes of mask m (1 i, 2 j,
+// 4 k; near[0]: the centre), whose terms are checked; the products multiply `slots` sums, sum s of
+// count[s] values with coefficient c[first[s]].  Left off (false) for coefficients so uneven that many
+// bricks of ordinary values would fail the check and run in FP64, and for stencils whose
+// coefficients after the first are all powers of two (the 7-point Laplacian): their products are
+// exact, so the FP64 chain rounds exactly as the reference's CPU code does, which callers that
+// compare cancelling sums with it rely on.
+static bool fx_table(const double *c, int n, const int (*near)[9], int masks, int slots, const int *first,
+                     const int *count, int xb, bool one, FxTab *t) {
+  t->on = 0;
+  double sum = 0.0, most = 0.0, heads = 0.0;
+  bool exact = true;  // c[k] x exact for every k > 0
+  for (int k = 0; k < n; ++k) {
+    sum += fabs(c[k]);
+    most = fmax(most, fabs(c[k]));
+    int e;
+    if (k && c[k] != 0.0) exact = exact && fabs(frexp(c[k], &e)) == 0.5;
+  }
+  if (exact || !(sum > 1e-270) || !(sum < 1e270)) return false;
+  for (int s = 0; s < slots; ++s) heads += fabs(c[first[s]]);
+  auto high = [](double x) {
+    long long b;
+    memcpy(&b, &x, 8);
+    return (int)(b >> 32) & 0x7FFFFFFF;
+  };
+  // q: the sum of the slots' |ch| is 2^31 at most (a hundredth more leaves sum ch xl, below 2^62, its
+  // room), each |ch| below 2^31, and the sum of cl xh below 2^63 (|xh| <= count 2^(xb - 32); the low
+  // halves are different ones for another power of two)
+  double low = 0.0;
+  bool fits = false;
+  const int top = ilogb(ldexp(1.01, 300) / heads) - 300 + 63;
+  for (t->q = top; t->q > top - 5; --t->q) {
+    low = 0.0;
+    double weighted = 0.0;
+    for (int s = 0; s < slots; ++s) {
+      const long long C = llrint(ldexp(c[first[s]], t->q));
+      t->cl[s] = (int)(unsigned)(unsigned long long)C;
+      t->ch[s] = (int)((C - t->cl[s]) >> 32);
+      low += fabs((double)t->cl[s]);
+      weighted += count[s] * fabs((double)t->cl[s]);
+    }
+    fits = ldexp(most, t->q) < 9.2e18 && ldexp(weighted, xb - 32) < 9.2e18;
+    if (fits) break;
+  }
+  if (!fits) return false;
+  // weights of the checked terms: a term c x passes when the high words of x and of
+  // c / (2 error / (n 2^-53)), added as exponents with fractions, reach exponent E (the sum of two
+  // high words never exceeds the high word of the product, so this errs towards FP64).  error: of
+  // the sum made here, in units of 2^(E - 1022): cut values, rounded coefficients, one or two
+  // roundings of half a unit (one: FxAcc<true>), sum cl xl
+  const double error = ldexp(sum, -xb) + ldexp((double)n, -1 - t->q) + ldexp(one ? 0.5 : 1.0, 64 - t->q - xb) + ldexp(low, 31 - t->q - xb);
+  const double least = 2.0 * error / (n * ldexp(1.0, -53));
+  double bits = 0.0;
+  for (int m = 0; m < masks; ++m) {
+    double x = fabs(c[near[m][0]]);
+    for (int k = 1; near[m][k] >= 0; ++k) x = fmin(x, fabs(c[near[m][k]]));
+    t->w[m] = x > 0.0 ? high(x) - high(least) - 2 : -(1 << 30);
+    if (masks == 8 || (m & (m - 1)) == 0) bits += fmax(0.0, t->w[m] / 1048576.0 + 1.0);
+  }
+  // uniform values: a point fails with probability about 2^-bits, one of a brick's 512 points with
+  // 2^(9 - bits); a brick in FP64 costs about three in fixed point
+  if (bits < 13.0) return false;
+  // sums of magnitude 1 .. 2^63 scale to normal numbers
+  const int s0 = 64 + 1 - xb - t->q;  // biased exponent of a sum of 1: E + s0
+  t->elo = 1 - s0 > 72 ? 1 - s0 : 72;
+  t->ehi = 2046 - s0 - 63 < 2046 ? 2046 - s0 - 63 : 2046;
+  return t->elo <= t->ehi;
+}
+
+// fx_table of a star or cube in kernel order (tp->c).
+static void fx_analyze(int fam, int r, int n, bool full, Taps *tp) {
+  tp->fx.on = 0;
+  const int w = 2 * r + 1;
+  auto pos = [&](int k, int j, int i) {
+    return fam == FAM_STAR ? star_index(k, j, i) : ((k + r) * w + (j + r)) * w + (i + r);
+  };
+  int near[8][9], first[FX_TAPS], count[FX_TAPS], slots = 0;
+  for (int m = 0; m < 8; ++m) {
+    int k = 0;
+    if (fam == FAM_CUBE || (m & (m - 1)) == 0)
+      for (int s = 0; s < 8; ++s)
+        if ((s & ~m) == 0)  // signs of the mask's axes
+          near[m][k++] = pos(m & 4 ? (s & 4 ? -1 : 1) : 0, m & 2 ? (s & 2 ? -1 : 1) : 0, m & 1 ? (s & 1 ? -1 : 1) : 0);
+    near[m][k++] = fam == FAM_CUBE || (m & (m - 1)) == 0 ? -1 : 0;
+    near[m][k < 9 ? k : 8] = -1;
+  }
+  bool rings = fam == FAM_STAR;  // one coefficient per ring of six
+  for (int t = 1; t < n && rings; ++t) rings = tp->c[t] == tp->c[6 * ((t - 1) / 6) + 1];
+  if (fam == FAM_CUBE && r == 2) {
+    if (!full) return;
+    // classes by sorted distances: (0,0,0) (0,0,1) (0,0,2) (0,1,1) (0,1,2) (0,2,2) (1,1,1) (1,1,2) (1,2,2) (2,2,2)
+    for (int a = 0; a <= 2; ++a)
+      for (int b = a; b <= 2; ++b)
+        for (int d = b; d <= 2; ++d) {
+          first[slots] = pos(a, b, d);
+          const int orders = a == b && b == d ? 1 : (a == b || b == d) ? 3 : 6;
+          count[slots++] = orders * (a ? 2 : 1) * (b ? 2 : 1) * (d ? 2 : 1);
+        }
+  } else if (rings) {
+    for (slots = 0; slots <= r; ++slots) {
+      first[slots] = slots ? 6 * slots - 5 : 0;
+      count[slots] = slots ? 6 : 1;
+    }
+  } else {
+    if (n > FX_TAPS) return;
+    for (slots = 0; slots < n; ++slots) {
+      first[slots] = slots;
+      count[slots] = 1;
+    }
+  }
+  if (fx_table(tp->c, n, near, fam == FAM_CUBE ? 8 : 5, slots, first, count, fam == FAM_CUBE && r == 2 ? 58 : 60,
+               fam == FAM_STAR && r == 1, &tp->fx))
+    tp->fx.on = slots < n ? 2 : 1;
 }
 
 // Classify a tap list and lay its coefficients out in kernel order.
@@ -136,6 +253,13 @@ static int analyze(const bk_stencil *st, const Layout &L, SweepPlan *plan, Taps 
     }
   }
   for (int t = 0; t < TAP_PAIRS; ++t) tp->cp[t] = make_float2(tp->cf[t], tp->cf[t]);
+  tp->fx.on = 0;
+  // 8x8x8 row-major bricks: stars, the radius-1 cube without mirror symmetry (with it the FP64 class
+  // sums take 14 operations per point, fewer cycles than 27 products here) and the radius-2 cube with one
+  // coefficient per sorted distance
+  if (plan->shape == 0 && !plan->ops &&
+      (fam == FAM_STAR || (fam == FAM_CUBE && r == 1 && !plan->sym) || (fam == FAM_CUBE && r == 2 && plan->sym && tp->kj && plan->symij)))
+    fx_analyze(fam, r, n, fam == FAM_CUBE && r == 2, tp);
   return BK_OK;
 }
 

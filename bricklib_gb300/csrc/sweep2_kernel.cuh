@@ -174,7 +174,11 @@ struct Sweep2Cfg {
   static constexpr int EI = CS4 ? (ES == 4 ? (SWZ ? 16 : 20) : 24)
                           : PERM ? (NEED % 8 <= 4 ? NEED - NEED % 8 + 4 : NEED - NEED % 8 + 12)
                                  : conflict_free_row(NEED, BI, ES, VE);
-  static constexpr int TILE = EK * EJ * EI;  // elements per brick tile
+  // the 125-point cube in fixed point: planes two elements longer, so that a quarter warp's pair loads
+  // from four rows of two planes fall in different banks
+  static constexpr bool FX125 = FAM == FAM_CUBE && R == 2 && ACC == ACCM_FXS;
+  static constexpr int SK = EJ * EI + (FX125 ? 2 : 0);  // elements per plane
+  static constexpr int TILE = EK * SK;                  // elements per brick tile
   // position within tile row jj of column ii (SWZ: the row's 16-byte units permuted)
   static __host__ __device__ __forceinline__ int col(int jj, int ii) {
     return SWZ ? ((((ii >> 2) ^ ((jj >> 1) & 3)) << 2) | (ii & 3)) : ii;
@@ -206,22 +210,27 @@ struct Sweep2Cfg {
   static constexpr int FTILE_BYTES = 0;
   // bricks per CTA: as many as fit 128 threads and a ~100 KB shared-memory budget
   static constexpr int PER_BRICK = 2 * TILE_BYTES + FTILE_BYTES + 3 * 36 * 4;
-  static constexpr int NB = CS4 ? 1 : PAIR ? PAIR_NB : cmax(1, cmin(cmax(1, 128 / TPB), (100 * 1024) / PER_BRICK));
+  static constexpr int NB = CS4 || FX125 ? 1 : PAIR ? PAIR_NB : cmax(1, cmin(cmax(1, 128 / TPB), (100 * 1024) / PER_BRICK));
   static constexpr int NT = TPB * NB;
   // native FP64 arithmetic on register operands (F64Ops).  Stars and cubes read them from a
   // shared-memory block after the tiles and the adjacency slots (F64Ops head, then the taps'
   // coefficients); the class-sum streams read them from the kernel parameters (a block would cost
   // them a resident CTA per SM, and they measured the same either way).
-  static constexpr bool F64R = ES == 8 && ACC == ACCM_NATIVE;
+  // (the fixed-point modes keep the block for the bricks they compute in FP64)
+  static constexpr bool FX = ACC == ACCM_FX || ACC == ACCM_FXS;
+  static constexpr bool F64R = ES == 8 && (ACC == ACCM_NATIVE || FX);
   static constexpr bool SYMF = FAM == FAM_CUBESYM || FAM == FAM_CUBESYM_IJ;
-  static constexpr bool F64S = F64R && (FAM == FAM_STAR || FAM == FAM_CUBE);
+  static constexpr bool F64S = F64R && (FAM == FAM_STAR || FAM == FAM_CUBE) && !FX125;
   static constexpr int NCOEF = FAM == FAM_STAR ? 1 + 6 * R : (2 * R + 1) * (2 * R + 1) * (2 * R + 1);
   static constexpr int COEFB = F64S ? ((F64Ops::NHEAD + NCOEF) * 8 + 15) / 16 * 16 : 0;
-  static constexpr int SMEM = NB * PER_BRICK + COEFB;
+  static constexpr int SCANB = FX ? 2 * NB * 2 * 8 : 0;  // fixed-point scans, [call parity][brick][warp] int2
+  static constexpr int SMEM = NB * PER_BRICK + COEFB + SCANB;
   // resident CTAs asked of the register allocator: the native FP32 / BF16 class-sum stream
   // (one warp per CTA) at <= 170 registers fits three warps per scheduler (12 per SM), which its
   // shared memory also allows; the compensated stream (two warps per CTA): BK_CS_COMP_MINB
-  static constexpr int MINB = CS4 ? (ACC == ACCM_NATIVE ? 12 : BK_CS_COMP_MINB) : 0;
+  // the fixed-point cubes: radius 1 five CTAs of two bricks (256^3: 236 us; four 244, three 261),
+  // the 125-point one six of one brick (298 us; seven 301 with fewer registers)
+  static constexpr int MINB = CS4 ? (ACC == ACCM_NATIVE ? 12 : BK_CS_COMP_MINB) : FX125 ? 6 : FX && FAM == FAM_CUBE ? 5 : 0;
 };
 
 // Tile coordinates (kk, jj, ii) of plan vector g for the star / cube neighbourhood.
@@ -323,7 +332,7 @@ __device__ __forceinline__ unsigned plan_entry(int g) {
   const int lk = kk - R - qk * BK, lj = jj - R - qj * BJ, li = ii - C::RP - qi * BI;
   const unsigned slot = (unsigned)((qk + 1) * 9 + (qj + 1) * 3 + (qi + 1));
   const unsigned src = (unsigned)((lk * BJ + lj) * BI + li);
-  const unsigned dst = (unsigned)((kk * C::EJ + jj) * C::EI + C::col(jj, ii));
+  const unsigned dst = (unsigned)(kk * C::SK + jj * C::EI + C::col(jj, ii));
   return slot | (src << 5) | (dst << 18);
 }
 
@@ -1179,6 +1188,96 @@ __device__ __forceinline__ void sweep2_brick(const T *rt, T *out_brick, int lt, 
   }
 }
 
+// One (j, i) column of a brick under the 125-point cube with one coefficient per sorted distance, in
+// FP64 on pair sums (58.5 operations per point), for the bricks not computed in fixed point.
+template <typename C>
+__device__ __forceinline__ void sym_cube_column_f64(const double *rt, double *ob, const int lt, const Taps &tp) {
+  constexpr int R = 2, SK = C::SK, SJ = C::EI;
+  const F64Ops f = F64Ops::load(tp);
+  const double *col = rt + ((lt >> 3) + R) * SJ + (lt & 7) + C::RP;
+  double acc[8];
+#pragma unroll 1
+  for (int cls = 0; cls < 6; ++cls) {  // (b, a) = (0,0) (0,1) (1,1) (0,2) (1,2) (2,2)
+    const int a = cls < 1 ? 0 : cls < 3 ? 1 : 2, b = cls == 2 || cls == 4 ? 1 : cls == 5 ? 2 : 0;
+    const double c0 = f64_coef(tp, sym_index(0, b, a, R)), c1 = f64_coef(tp, sym_index(1, b, a, R)),
+                 c2 = f64_coef(tp, sym_index(2, b, a, R));
+    double q[12];
+#pragma unroll
+    for (int kk = 0; kk < 12; ++kk) {
+      const double *c = col + kk * SK;
+      auto four = [&](int x, int y) {  // rows -+x, columns -+y, each value once
+        const double lo = y ? f.add(c[-x * SJ - y], c[-x * SJ + y]) : c[-x * SJ];
+        if (x == 0) return lo;
+        return f.add(lo, y ? f.add(c[x * SJ - y], c[x * SJ + y]) : c[x * SJ]);
+      };
+      q[kk] = a == b ? four(b, a) : f.add(four(b, a), four(a, b));
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const double v = cls ? fma(c0, q[k + 2], acc[k]) : f.mul(c0, q[k + 2]);
+      acc[k] = fma(c2, f.add(q[k], q[k + 4]), fma(c1, f.add(q[k + 1], q[k + 3]), v));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) store_stream(ob + k * 64 + lt, acc[k]);
+}
+
+// A converted brick's outputs in fixed point (fx.cuh).
+template <typename T, int R, int FAM, int ACC>
+__device__ __forceinline__ void sweep2_brick_fx(const double *rt, double *out_brick, int lt, const Taps &tp, int E) {
+  typedef Sweep2Cfg<T, 8, 8, 8, R, FAM, ACC> C;
+  constexpr int SK = C::SK, SJ = C::EI;
+  if constexpr (C::FX125) {
+    // a row per thread; a quarter warp takes four rows of two planes
+    const int j = (lt & 3) | ((lt >> 1) & 4), k = ((lt >> 2) & 1) | ((lt >> 3) & 6);
+    const double *c = rt + (k + R) * SK + (j + R) * SJ;
+    double *o = out_brick + k * 64 + j * 8;
+    const bool two = (reinterpret_cast<uintptr_t>(o) & 15) == 0;
+    fx_cube125_row([&](int dk, int dj, int p) { return ld_pair(c + dk * SK + dj * SJ + 2 * p); },
+                   [&](int p, double y0, double y1) {
+                     if (two) st_pair(o + 2 * p, make_double2(y0, y1));
+                     else {
+                       store_stream(o + 2 * p, y0);
+                       store_stream(o + 2 * p + 1, y1);
+                     }
+                   },
+                   tp.fx, fx_scale<58>(E, tp.fx.q));
+    return;
+  } else {
+  // four planes of a column pair; a quarter warp takes rows two apart, which fall in different banks
+  const int q = (lt >> 2) & 7, j = (q & 4) | ((q & 1) << 1) | ((q >> 1) & 1), i = 2 * (lt & 3), k0 = 4 * (lt >> 5);
+  const double *c = rt + (k0 + R) * SK + (j + R) * SJ + i + C::RP;
+  double *o = out_brick + k0 * 64 + j * 8 + i;
+  const bool two = (reinterpret_cast<uintptr_t>(o) & 15) == 0;  // output bricks may start anywhere
+  auto put = [&](int k, double y0, double y1) {
+    if (two) st_pair(o + k * 64, make_double2(y0, y1));
+    else {
+      store_stream(o + k * 64, y0);
+      store_stream(o + k * 64 + 1, y1);
+    }
+  };
+  const int scale = fx_scale<60>(E, tp.fx.q);
+  if constexpr (FAM == FAM_STAR)
+    fx_star_pairs<R, ACC == ACCM_FXS>([&](int k, int dj, int m) { return ld_pair(c + k * SK + dj * SJ + 2 * m); },
+                                      [&](int k, int di) { return c[k * SK + di]; }, put, tp.fx, scale);
+  else
+    fx_cube_pairs([&](int k, int dj) { return ld_pair(c + k * SK + dj * SJ); },
+                  [&](int k, int dj, int di) { return c[k * SK + dj * SJ + di]; }, put, tp.fx, scale);
+  }
+}
+// A thread's share of a tile's values.
+template <typename C, int R, int FAM, bool SUM>
+__device__ __forceinline__ auto sweep2_share(int lt) {
+  auto at = [](int k, int j, int i) { return (k + R) * C::SK + (j + R) * C::EI + i + C::RP; };
+  if constexpr (FAM == FAM_STAR) {
+    const FxFaces<R, decltype(at)> f{lt, at};
+    return fx_share<true, false, SUM, false, 60>(lt, f, f);
+  } else {
+    const FxBox<R, decltype(at)> f(lt, at);
+    return fx_share<true, false, SUM, true, C::FX125 ? 58 : 60>(lt, f, f);
+  }
+}
+
 // IST: FP64 mirror-symmetric cubes streamed along i (sym_cube_istream): each CTA takes a
 // contiguous share of the list instead of every gridDim.x-th group.
 template <typename T, int BK, int BJ, int BI, int R, int FAM, int ACC, bool BATCH, bool IST>
@@ -1371,6 +1470,12 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
       csw[e] = e < F64Ops::NHEAD ? tp.one_mz[e] : tp.c[e - F64Ops::NHEAD];
   }
 
+  // fixed point: this thread's share of its brick's values, and the brick's scans by parity
+  const auto share = sweep2_share<C, R, C::FX ? FAM : FAM_STAR, ACC == ACCM_FXS>(lt);
+  int2 *scan = reinterpret_cast<int2 *>(smem_raw + NB * C::PER_BRICK + C::COEFB) + 2 * slot;
+  static_assert(!C::FX || (TPB == 64 && BK == 8 && BJ == 8 && BI == 8 && (FAM == FAM_STAR || FAM == FAM_CUBE)),
+                "fixed point: stars and cubes on 8x8x8 bricks, 64 threads each");
+
   // prologue: adjacency of the first two groups, copies of the first
   Walk w1{g0, 0};
   Walk w2 = advance(w1), w3 = advance(w2);  // the next group and the one after
@@ -1430,7 +1535,19 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
     } else if (active) {
       T *out = reinterpret_cast<T *>(*reinterpret_cast<const unsigned long long *>(nbr + 30));
       const size_t ostep = *reinterpret_cast<const unsigned long long *>(nbr + 34);
-      sweep2_brick<T, BK, BJ, BI, R, FAM, ACC>(rt, out + (size_t)nbr[13] * ostep, lt, tp, cs);
+      if constexpr (C::FX) {
+        int E = 0;
+        bool stopped = false;
+        double *tile = reinterpret_cast<double *>(const_cast<T *>(rt));
+        T *ob = out + (size_t)nbr[13] * ostep;
+        if (fx_prepare(share, tile, tile, tp.fx, scan + 2 * NB * cur, slot, E, true, false, stopped, [] {}))
+          sweep2_brick_fx<T, R, FAM, ACC>(tile, ob, lt, tp, E);
+        else if constexpr (C::FX125)
+          sym_cube_column_f64<C>(tile, reinterpret_cast<double *>(ob), lt, tp);
+        else
+          sweep2_brick<T, BK, BJ, BI, R, FAM, ACCM_NATIVE>(rt, ob, lt, tp, cs);
+      } else
+        sweep2_brick<T, BK, BJ, BI, R, FAM, ACC>(rt, out + (size_t)nbr[13] * ostep, lt, tp, cs);
     }
     store_adj(nfar);  // group it + 2; read after the next iteration's first barrier
   }

@@ -60,8 +60,17 @@ struct StarTmaCfg {
   // the FP64 register-operand block (F64Ops head, then NTAP coefficients; 8-byte aligned)
   static constexpr int NTAP = 1 + 6 * R;
   static constexpr int O_COEF = 64 + 4 * TMA_MAX_STAGES * NB + 16;
-  static constexpr int META = O_COEF + 8 * (F64Ops::NHEAD + NTAP);
-  static constexpr int smem(int stages) { return 128 + stages * NB * BRICK + META; }  // + base alignment slack
+  // ... and the fixed-point scans, [call parity][brick][warp] int2 (16-byte aligned)
+  static constexpr int O_SCAN = (O_COEF + 8 * (F64Ops::NHEAD + NTAP) + 15) / 16 * 16;
+  static constexpr int META = O_SCAN + 2 * NB * 2 * 8;
+  // fixed point of radius 1 and 2: a tile of integers per brick after the meta data (128-byte aligned)
+  static constexpr int fx_tile(int acc) {
+    return R <= 2 && ES == 8 && (acc == ACCM_FX || acc == ACCM_FXS) ? FxTile<R <= 2 ? R : 1>::SIZE * 8 : 0;
+  }
+  static constexpr int o_tile(int stages) { return (stages * NB * BRICK + META + 127) / 128 * 128; }
+  static constexpr int smem(int stages, int acc) {  // + base alignment slack
+    return 128 + (fx_tile(acc) ? o_tile(stages) + NB * fx_tile(acc) : stages * NB * BRICK + META);
+  }
 };
 
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
@@ -274,14 +283,15 @@ __device__ __forceinline__ void star_column(const unsigned char *buf, const int 
   }
 }
 
-// The native FP64 column: the same operations in the same order per point as star_column, on
-// register operands only (F64Ops; the coefficients cr read from shared memory once per thread),
-// with the loop over the column's BK points innermost, so that consecutive multiply-adds share
-// one coefficient and each takes its other factor straight from a shared-memory load.
+// The native FP64 column (bricks not computed in fixed point, and stencils that cannot be): the
+// same operations in the same order per point as star_column, on register operands only (F64Ops;
+// coefficient t read from shared memory at cs[t]), with the loop over the column's BK points
+// innermost, so that consecutive multiply-adds share one coefficient and each takes its other
+// factor straight from a shared-memory load.
 template <int BK, int BJ, int BI, int R>
 __device__ __forceinline__ void star_column_f64(const unsigned char *buf, const int cKL, const int cC, const int cKH,
                                                 const int (&oi)[2 * R], const int (&si)[2 * R], const int (&oj)[2 * R],
-                                                const int (&sj)[2 * R], double *ob, const double (&cr)[1 + 6 * R],
+                                                const int (&sj)[2 * R], double *ob, const double *cr,
                                                 const F64Ops &f64) {
   constexpr int PK = BJ * BI;
   const double *f = reinterpret_cast<const double *>(buf);
@@ -310,15 +320,143 @@ __device__ __forceinline__ void star_column_f64(const unsigned char *buf, const 
   for (int k = 0; k < BK; ++k) store_stream(ob + k * PK, acc[k]);
 }
 
+// star_column_f64 for thread l of a brick, on its staged regions; cs: the register-operand block.
+template <typename C, int R>
+__device__ __forceinline__ void star_column_f64_of(const double *buf, const int l, double *out, const double *cs) {
+  const int j = l >> 3, i = l & 7;
+  constexpr int eKL = C::O_KL / 8, eKH = C::O_KH / 8, eJL = C::O_JL / 8, eJH = C::O_JH / 8, eIL = C::O_IL / 8,
+                eIH = C::O_IH / 8, IW = C::IW;
+  int oi[2 * R], si[2 * R], oj[2 * R], sj[2 * R];
+#pragma unroll
+  for (int d = 1; d <= R; ++d)
+#pragma unroll
+    for (int sg = 0; sg < 2; ++sg) {
+      const int q = 2 * (d - 1) + sg, ii = sg ? i - d : i + d, jj = sg ? j - d : j + d;
+      oi[q] = ii >= 8 ? eIH + j * IW + ii - 8 : ii < 0 ? eIL + j * IW + IW + ii : j * 8 + ii;
+      si[q] = ii >= 8 || ii < 0 ? 8 * IW : 64;
+      oj[q] = jj >= 8 ? eJH + (jj - 8) * 8 + i : jj < 0 ? eJL + (R + jj) * 8 + i : jj * 8 + i;
+      sj[q] = jj >= 8 || jj < 0 ? R * 8 : 64;
+    }
+  star_column_f64<8, 8, 8, R>(reinterpret_cast<const unsigned char *>(buf), eKL + l, l, eKH + l, oi, si, oj, sj, out + l,
+                              cs + F64Ops::NHEAD, F64Ops::load(cs));
+}
+
+// The consumer threads of a fixed-point star sweep (fx.cuh): 64 threads (two warps) per brick.
+// Radius 1 and 2: the values are read from the stage into registers, the stage goes back to the
+// producer, and the integers go to a tile of their own, where every tap is at a constant distance
+// (a stage's faces each have strides of their own) and the next brick's copies run meanwhile.
+// Radius 4, whose tile would take 32 KB: in the stage, in place.
+template <typename C, int R, bool SUM>
+__device__ __forceinline__ void star_fx_consume(unsigned char *sm, const unsigned full0, const unsigned empty0,
+                                                const unsigned *outb, volatile int *abort_word, const int S,
+                                                const int bs, const int lt, const SweepArgs &a, const Taps &tp,
+                                                const long long ngroups, const unsigned long long lim) {
+  constexpr int NB = C::NB, IW = C::IW;
+  constexpr bool TILE = R <= 2;
+  static_assert(C::TPB == 64 && NB <= 2 && C::ES == 8, "8x8x8 bricks of FP64");
+  static_assert(C::O_KL == 4096 && C::BRICK == C::O_KL + 8 * (256 * R + 128 * IW), "faces one after the other");
+  const int lane = lt & 31;
+  int2 *scan = reinterpret_cast<int2 *>(sm + S * NB * C::BRICK + C::O_SCAN) + 2 * bs;
+  double *tile = reinterpret_cast<double *>(sm + C::o_tile(S) + bs * C::fx_tile(ACCM_FX));
+  const auto share = [&] {
+    const FxDense<R, IW> dense{lt};
+    if constexpr (TILE) return fx_share<true, true, SUM, false, 60>(lt, dense, FxTile<R>(lt));
+    else return fx_share<true, true, SUM, false, 60>(lt, dense, dense);
+  }();
+  // this thread's column pair and four planes.  In the tile a quarter warp takes rows two apart
+  const int q8 = (lt >> 2) & 7, pi = 2 * (lt & 3), pk = 4 * (lt >> 5);
+  const int pj = TILE ? FxTile<TILE ? R : 1>::row(lt) : q8;
+  int st = 0;
+  unsigned ph = 0;   // phase parity of the stage's current use
+  unsigned par = 0;  // parity of the CTA's groups (scans)
+  for (long long g = blockIdx.x; g < ngroups; g += gridDim.x, par ^= 1u) {
+    const bool ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(full0 + 8 * st, ph, lim));
+    if (!ok) {
+      atomicOr(a.err, FLAG_TIMEOUT);
+      *abort_word = 1;
+    }
+    const unsigned ob_idx = outb[st * NB + bs];
+    const bool active = ok && ob_idx != 0xFFFFFFFFu;
+    double *buf = reinterpret_cast<double *>(sm + (st * NB + bs) * C::BRICK);
+    auto release = [&] {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty0 + 8 * st);
+    };
+    int E = 0;
+    bool stopped = false;
+    // (a thread that gives up says so at the brick's first barrier, and its 64 threads stop)
+    const bool fx = fx_prepare(share, buf, TILE ? tile : buf, tp.fx, scan + 2 * NB * par, bs, E, active, !ok, stopped,
+                               [&] {
+                                 if constexpr (TILE) release();
+                               });
+    if (stopped) break;
+    if (active) {
+      double *out = reinterpret_cast<double *>(a.out) + a.out_off + (size_t)ob_idx * a.out_step;
+      if (fx) {
+        double *o = out + pk * 64 + pj * 8 + pi;
+        const bool two = (reinterpret_cast<uintptr_t>(o) & 15) == 0;  // output bricks may start anywhere
+        auto put = [&](int k, double y0, double y1) {
+          if (two) st_pair(o + k * 64, make_double2(y0, y1));
+          else {
+            store_stream(o + k * 64, y0);
+            store_stream(o + k * 64 + 1, y1);
+          }
+        };
+        const int scale = fx_scale<60>(E, tp.fx.q);
+        if constexpr (TILE) {
+          typedef FxTile<R> X;
+          const double *c = tile + X::at(pk, pj, pi);
+          fx_star_pairs<R, SUM>([&](int k, int dj, int m) { return ld_pair(c + k * X::SK + dj * X::SJ + 2 * m); },
+                                [&](int k, int di) { return c[k * X::SK + di]; }, put, tp.fx, scale);
+        } else {
+          auto at = [&](int k, int j, int i) {  // one of the coordinates may lie in a face
+            return k < 0    ? 512 + ((k + R) * 8 + j) * 8 + i
+                   : k >= 8 ? 512 + 64 * R + ((k - 8) * 8 + j) * 8 + i
+                   : j < 0  ? 512 + 128 * R + (k * R + j + R) * 8 + i
+                   : j >= 8 ? 512 + 192 * R + (k * R + j - 8) * 8 + i
+                   : i < 0  ? 512 + 256 * R + (k * 8 + j) * IW + IW + i
+                   : i >= 8 ? 512 + 256 * R + 64 * IW + (k * 8 + j) * IW + i - 8
+                            : (k * 8 + j) * 8 + i;
+          };
+          fx_star_pairs<R, SUM>([&](int k, int dj, int m) { return ld_pair(buf + at(pk + k, pj + dj, pi + 2 * m)); },
+                                [&](int k, int di) { return buf[at(pk + k, pj, pi + di)]; }, put, tp.fx, scale);
+        }
+      } else {
+        // FP64: one column per thread; its offsets are found here (kept out of the loop's registers)
+        int l = lt;
+        asm volatile("" : "+r"(l));
+        star_column_f64_of<C, R>(buf, l, out, reinterpret_cast<const double *>(sm + S * NB * C::BRICK + C::O_COEF));
+      }
+    }
+    if (!(TILE && fx)) {
+      // an in-place conversion wrote the stage through the generic proxy; order those writes before
+      // the copies that refill it
+      if constexpr (!TILE) fence_proxy_async_smem();
+      release();
+    }
+    if (++st == S) {
+      st = 0;
+      ph ^= 1u;
+    }
+  }
+}
+
+// Resident CTAs asked of the register allocator for the fixed-point stars (radius 1, 2 and 4: 96, 120
+// and 128 registers).  256^3, us, with one CTA less / these / one more: 7-point star with one ring
+// coefficient 80 / 76 / 81, 13-point 117 / 104 / 117, 25-point 237 / 174 / --.
+constexpr int star_tma_minb(int r, int acc) {
+  return acc == ACCM_FX || acc == ACCM_FXS ? (r == 1 ? 4 : 3) : 0;
+}
+
 template <typename T, int BK, int BJ, int BI, int R, int ACC, bool NI>
-__global__ void __launch_bounds__(StarTmaCfg<T, BK, BJ, BI, R, NI>::NT)
+__global__ void __launch_bounds__(StarTmaCfg<T, BK, BJ, BI, R, NI>::NT, star_tma_minb(R, ACC))
 sweep_star_tma_kernel(const __grid_constant__ TmaMaps maps, const SweepArgs a, const Taps tp, const int S) {
   typedef StarTmaCfg<T, BK, BJ, BI, R, NI> C;
   typedef typename Elem<T>::acc AT;
   constexpr int NB = C::NB, TPB = C::TPB, IW = C::IW, PK = BJ * BI;
   static_assert(7 * NB <= 32, "one producer lane per (brick, region)");
   static_assert(TPB % 32 == 0, "whole warps per brick");
-  static_assert(C::ES == 8 || ACC != ACCM_FF, "float-float needs FP64 storage");
+  static_assert(C::ES == 8 || (ACC != ACCM_FF && ACC != ACCM_FX && ACC != ACCM_FXS), "FP64 storage");
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const unsigned raw = smem_u32(smem_raw);
@@ -443,6 +581,10 @@ sweep_star_tma_kernel(const __grid_constant__ TmaMaps maps, const SweepArgs a, c
 
   // -------------------------------------------------------------------- consumer warps
   const int bs = threadIdx.x / TPB, lt = threadIdx.x - bs * TPB;
+  if constexpr (ACC == ACCM_FX || ACC == ACCM_FXS) {
+    star_fx_consume<C, R, ACC == ACCM_FXS>(sm, full0, empty0, outb, abort_word, S, bs, lt, a, tp, ngroups, lim);
+    return;
+  }
   const int j = lt / BI, i = lt - j * BI;
   // per-lane shared-memory element offsets (from the brick's stage buffer) and k strides
   // of the i and j taps: index 2(d-1) is +d, 2(d-1)+1 is -d
@@ -470,7 +612,6 @@ sweep_star_tma_kernel(const __grid_constant__ TmaMaps maps, const SweepArgs a, c
 #pragma unroll
   for (int t = 0; t < C::NTAP; ++t) cr[t] = F64R ? coef_s[F64Ops::NHEAD + t] : 0.0;
   const F64Ops f64 = F64R ? F64Ops::load(coef_s) : F64Ops{0.0, 0.0};
-
   int st = 0;
   unsigned ph = 0;  // phase parity of the stage's current use
   for (long long g = g0; g < ngroups; g += gstep) {
@@ -535,7 +676,7 @@ int launch_star_tma(const SweepArgs &a, const Taps &tp, int dtype, cudaStream_t 
   // default depth 2: on GB300 more resident CTAs beat deeper pipelines (FP32 star7 at 512^3:
   // 602 / 490 GStencil/s with 2 / 3 stages)
   const int S = tma_stages(2);
-  const int smem = C::smem(S);
+  const int smem = C::smem(S, ACC);
   if (smem > 227 * 1024) return fail(BK_ERR_UNSUPPORTED, "TMA sweep stage buffers exceed shared memory");
   TmaMaps maps;
   if (!star_tma_maps(a, dtype, BK, BJ, BI, R, C::IW, &maps)) return fail(BK_ERR_UNSUPPORTED, "field not describable to the TMA unit");

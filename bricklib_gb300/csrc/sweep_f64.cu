@@ -39,6 +39,17 @@ namespace bk {
 int sweep_dispatch_f64(const SweepPlan &p, const SweepArgs &a, Taps &tp, cudaStream_t s) {
   if (p.v2) {
     if (p.shape == 0) {
+      // fixed point where the stencil allows it (BK_SWEEP_ISTREAM=0 asks for the FP64 pair sums)
+      if (p.acc == ACCM_NATIVE && tp.fx.on && (p.fam != FAM_CUBE || p.r == 1 || p.istream)) {
+#define BK_FX(R_, FAM_, ACC_) \
+  if (p.r == R_ && p.fam == FAM_) return launch_sweep2<double, 8, 8, 8, R_, FAM_, ACC_>(a, tp, s);
+        if (tp.fx.on == 2) {
+          BK_FX(1, FAM_STAR, ACCM_FXS) BK_FX(2, FAM_STAR, ACCM_FXS) BK_FX(4, FAM_STAR, ACCM_FXS) BK_FX(2, FAM_CUBE, ACCM_FXS)
+        } else {
+          BK_FX(1, FAM_STAR, ACCM_FX) BK_FX(2, FAM_STAR, ACCM_FX) BK_FX(4, FAM_STAR, ACCM_FX) BK_FX(1, FAM_CUBE, ACCM_FX)
+        }
+#undef BK_FX
+      }
       // mirror-symmetric cubes: pair sums, fewer multiply-adds
       if (p.sym && p.fam == FAM_CUBE && p.acc == ACCM_NATIVE && p.istream) {
         if (p.r == 1) return launch_sweep2<double, 8, 8, 8, 1, FAM_CUBESYM, ACCM_NATIVE, false, true>(a, tp, s);
@@ -70,6 +81,16 @@ int sweep_dispatch_f64(const SweepPlan &p, const SweepArgs &a, Taps &tp, cudaStr
   if (p.fam == FAM_GENERIC)
     for (int t = 0; t < tp.n; ++t) tp.toff[t] = p.toff1[t];
   if (p.shape == 0) {
+    if (p.acc == ACCM_NATIVE && p.fam == FAM_STAR && tp.fx.on && !p.ops) {  // the bits of the other star kernels
+#define BK_FX(R_, ACC_) \
+  if (p.r == R_) return launch_sweep<double, 8, 8, 8, R_, FAM_STAR, true, ACC_>(a, tp, s);
+      if (tp.fx.on == 2) {
+        BK_FX(1, ACCM_FXS) BK_FX(2, ACCM_FXS) BK_FX(4, ACCM_FXS)
+      } else {
+        BK_FX(1, ACCM_FX) BK_FX(2, ACCM_FX) BK_FX(4, ACCM_FX)
+      }
+#undef BK_FX
+    }
     BK_SHAPE_SET(8, 8, 8, ACCM_NATIVE)
     BK_SHAPE_SET(8, 8, 8, ACCM_FF)
   } else if (p.shape == 1) {

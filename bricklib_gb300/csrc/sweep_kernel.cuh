@@ -15,7 +15,7 @@
 // generic family.
 #pragma once
 
-#include "bk_common.cuh"
+#include "fx.cuh"
 
 namespace bk {
 
@@ -28,7 +28,10 @@ enum Family { FAM_GENERIC = 0, FAM_STAR = 1, FAM_CUBE = 2, FAM_CUBESYM = 3, FAM_
 __host__ __device__ constexpr int sym_index(int ak, int aj, int ai, int r) {
   return 200 + (ak * (r + 1) + aj) * (r + 1) + ai;
 }
-enum AccMode { ACCM_NATIVE = 0, ACCM_COMP = 1, ACCM_FF = 2 };
+// ACCM_FX / ACCM_FXS: native FP64 sums of 8x8x8 bricks in fixed point (fx.cuh); FXS: star rings
+// of one coefficient each, added before they are multiplied.  Chosen by the stencil (Taps::fx),
+// never asked for by a caller.
+enum AccMode { ACCM_NATIVE = 0, ACCM_COMP = 1, ACCM_FF = 2, ACCM_FX = 3, ACCM_FXS = 4 };
 
 // One domain of a batch (device table entry).
 struct BatchDomain {
@@ -84,6 +87,7 @@ struct Taps {
   // {1.0, -0.0}, which the native FP64 kernels hold in registers (F64Ops); set by the host so
   // that the compiler cannot fold them back into plain additions and products
   double one_mz[2];
+  FxTab fx;
 };
 
 __host__ __device__ constexpr int sweep_threads(int tpb) { return tpb < 128 ? 128 : tpb; }
@@ -365,6 +369,10 @@ __device__ __forceinline__ AT stencil_point(const AT *__restrict__ c, const Taps
   }
 }
 
+// Byte position of the fixed-point scans: after the tiles (TILES bytes) and the adjacency slots.
+template <size_t TILES, int NB>
+constexpr size_t SWEEP_SCAN_AT = (TILES + sizeof(unsigned) * 28 * NB + 15) / 16 * 16;
+
 template <typename T, int BK, int BJ, int BI, int R, int FAM, bool RM, int ACC>
 __global__ void __launch_bounds__(sweep_threads(BJ * BI))
 sweep_kernel(const SweepArgs a, const Taps tp) {
@@ -384,6 +392,11 @@ sweep_kernel(const SweepArgs a, const Taps tp) {
   unsigned *nbr = nbrs + slot * 28;
   const T *in = reinterpret_cast<const T *>(a.in) + a.in_off;
   T *out = reinterpret_cast<T *>(a.out) + a.out_off;
+
+  // fixed point (fx.cuh): the brick's scans, [warp] int2 behind the adjacency slots
+  constexpr bool FX = ACC == ACCM_FX || ACC == ACCM_FXS;
+  static_assert(!FX || (TPB == 64 && BK == 8 && RM && FAM == FAM_STAR), "fixed point: stars on 8x8x8 bricks");
+  int2 *scan = reinterpret_cast<int2 *>(smem_raw + SWEEP_SCAN_AT<sizeof(AT) * TILE * NB, NB>) + 2 * slot;
 
   for (long long base = (long long)blockIdx.x * NB; base < a.nlist; base += (long long)gridDim.x * NB) {
     const long long n = base + slot;
@@ -423,7 +436,36 @@ sweep_kernel(const SweepArgs a, const Taps tp) {
       }
     }
     __syncthreads();
-    if (active) {
+    bool done = false;
+    if constexpr (FX) {
+      if (active) {
+        auto at = [](int k, int j, int i) { return ((k + R) * EJ + j + R) * EI + i + R; };
+        int E = 0;
+        bool stopped = false;
+        const FxFaces<R, decltype(at)> f{lt, at};
+        done = fx_prepare(fx_share<false, false, ACC == ACCM_FXS, false, 60>(lt, f, f), tile, tile, tp.fx, scan, slot, E, true,
+                          false, stopped, [] {});
+        if (done) {
+          const int j = (lt >> 2) & 7, i = 2 * (lt & 3);
+          const int k0 = 4 * (lt >> 5);
+          const AT *c = tile + at(k0, j, i);
+          T *ob = out + (size_t)nbr[13] * a.out_step + (k0 * BJ + j) * BI + i;
+          constexpr int SK = EJ * EI;
+          fx_star_pairs<R, ACC == ACCM_FXS>(
+              [&](int k, int dj, int m) {
+                const AT *x = c + k * SK + dj * EI + 2 * m;
+                return make_double2(x[0], x[1]);
+              },
+              [&](int k, int di) { return c[k * SK + di]; },
+              [&](int k, double y0, double y1) {
+                ob[k * TPB] = y0;
+                ob[k * TPB + 1] = y1;
+              },
+              tp.fx, fx_scale<60>(E, tp.fx.q));
+        }
+      }
+    }
+    if (active && !done) {
       const int j = lt / BI, i = lt - (lt / BI) * BI;
       T *ob = out + (size_t)nbr[13] * a.out_step;
 #pragma unroll 1
@@ -431,7 +473,7 @@ sweep_kernel(const SweepArgs a, const Taps tp) {
         const AT *c = tile + ((k + R) * EJ + (j + R)) * EI + (i + R);
         typename Elem<T>::acc v;
         if constexpr (ACC == ACCM_FF) v = stencil_point_ff<EJ, EI, R, FAM>(c, tp);
-        else v = stencil_point<AT, EJ, EI, R, FAM, ACC>(c, tp);
+        else v = stencil_point<AT, EJ, EI, R, FAM, FX ? ACCM_NATIVE : ACC>(c, tp);
         const int o = RM ? (k * BJ + j) * BI + i : a.L.offset(k, j, i);
         Elem<T>::store(ob + o, op_apply(v, tp.post));
       }
@@ -447,7 +489,9 @@ int launch_sweep(const SweepArgs &a, const Taps &tp, cudaStream_t s) {
   constexpr int NT = sweep_threads(TPB);
   constexpr int NB = NT / TPB;
   constexpr int TILE = (BK + 2 * R) * (BJ + 2 * R) * (BI + 2 * R);
-  constexpr size_t smem = sizeof(AT) * TILE * NB + sizeof(unsigned) * 28 * NB;
+  constexpr bool FX = ACC == ACCM_FX || ACC == ACCM_FXS;
+  constexpr size_t smem = FX ? SWEEP_SCAN_AT<sizeof(AT) * TILE * NB, NB> + 16 * NB
+                             : sizeof(AT) * TILE * NB + sizeof(unsigned) * 28 * NB;
   static_assert(smem <= 227 * 1024, "tile too large");
   auto kern = sweep_kernel<T, BK, BJ, BI, R, FAM, RM, ACC>;
   if (smem > 48 * 1024) {

@@ -130,6 +130,16 @@ int sweep_dispatch_tma(const SweepPlan &p, const SweepArgs &a, Taps &tp, cudaStr
     return fail(BK_ERR_UNSUPPORTED, "the TMA sweep covers star stencils on row-major 8x8x8 bricks");
   switch (p.dtype) {
     case BK_F64:
+      if (p.acc == ACCM_NATIVE && tp.fx.on) {
+#define BK_FX_CASE(R_, ACC_) \
+  if (p.r == R_) return launch_star_tma<double, 8, 8, 8, R_, ACC_, true>(a, tp, p.dtype, s);
+        if (tp.fx.on == 2) {
+          BK_FX_CASE(1, ACCM_FXS) BK_FX_CASE(2, ACCM_FXS) BK_FX_CASE(4, ACCM_FXS)
+        } else {
+          BK_FX_CASE(1, ACCM_FX) BK_FX_CASE(2, ACCM_FX) BK_FX_CASE(4, ACCM_FX)
+        }
+#undef BK_FX_CASE
+      }
       BK_TMA_RADII(double, ACCM_NATIVE)
       BK_TMA_RADII(double, ACCM_FF)
       break;
