@@ -235,6 +235,17 @@ int batch_dispatch(const BatchStencil &bs, const BatchDomain *doms, unsigned ndo
   BK_B2(BK_, BJ_, BI_, 1, FAM_STAR) BK_B2(BK_, BJ_, BI_, 2, FAM_STAR) BK_B2(BK_, BJ_, BI_, 4, FAM_STAR) \
   BK_B2(BK_, BJ_, BI_, 1, FAM_CUBE) BK_B2(BK_, BJ_, BI_, 2, FAM_CUBE)
     if (p.shape == 0) {
+      // fixed point where the stencil allows it, as the plain sweep (the same bits)
+      if constexpr (sizeof(T) == 8 && ACC == ACCM_NATIVE) {
+#define BK_FX(R_, FAM_, ACC_) \
+  if (p.r == R_ && p.fam == FAM_) return launch_sweep2<T, 8, 8, 8, R_, FAM_, ACC_, true>(a, tp, s, grid_cap);
+        if (tp.fx.on == 2) {
+          BK_FX(1, FAM_STAR, ACCM_FXS) BK_FX(2, FAM_STAR, ACCM_FXS) BK_FX(4, FAM_STAR, ACCM_FXS) BK_FX(2, FAM_CUBE, ACCM_FXS)
+        } else if (tp.fx.on == 1) {
+          BK_FX(1, FAM_STAR, ACCM_FX) BK_FX(2, FAM_STAR, ACCM_FX) BK_FX(4, FAM_STAR, ACCM_FX) BK_FX(1, FAM_CUBE, ACCM_FX)
+        }
+#undef BK_FX
+      }
       if constexpr ((sizeof(T) <= 4 && (ACC == ACCM_NATIVE || ACC == ACCM_COMP)) || (sizeof(T) == 8 && ACC == ACCM_NATIVE)) {
         // mirror-symmetric cubes: the class sums streamed along each domain's runs of bricks, as
         // the plain sweep streams them (the same bits as the plain sweep of the same bricks)

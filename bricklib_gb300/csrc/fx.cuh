@@ -44,6 +44,9 @@ struct FxTab {
   int q;                         // C = c 2^q
 };
 
+bool fx_table(const double *c, int n, const int (*near)[9], int masks, int slots, const int *first, const int *count,
+              int xb, bool one, FxTab *t);
+
 // What a thread learns of its share of a brick's values, and after the exchange the whole brick's.
 struct FxScan {
   unsigned top;  // largest high word without sign

@@ -37,8 +37,8 @@ static int shape_of(const Layout &L) {
 // coefficients after the first are all powers of two (the 7-point Laplacian): their products are
 // exact, so the FP64 chain rounds exactly as the reference's CPU code does, which callers that
 // compare cancelling sums with it rely on.
-static bool fx_table(const double *c, int n, const int (*near)[9], int masks, int slots, const int *first,
-                     const int *count, int xb, bool one, FxTab *t) {
+bool fx_table(const double *c, int n, const int (*near)[9], int masks, int slots, const int *first, const int *count,
+              int xb, bool one, FxTab *t) {
   t->on = 0;
   double sum = 0.0, most = 0.0, heads = 0.0;
   bool exact = true;  // c[k] x exact for every k > 0

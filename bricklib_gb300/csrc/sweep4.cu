@@ -7,8 +7,10 @@
 // a 16-byte copy where a block of a tile row's centre (or a whole i halo) is consecutive and
 // aligned in its brick, else one copy per element.  Out-of-range list entries, and out-of-range
 // adjacency entries in the slots the tile reads, are clamped / skipped and raise the device error
-// flag, as in the 3-D kernels.
-#include "bk_common.cuh"
+// flag, as in the 3-D kernels.  Radius-1 stars on FP64 storage are summed in fixed point (fx.cuh).
+#include <cstring>
+
+#include "fx.cuh"
 
 namespace bk {
 
@@ -33,6 +35,7 @@ struct Taps4 {
   double c[BK_MAX_TAPS4];
   float cf[BK_MAX_TAPS4];
   double mzero;  // -0.0: the addend that makes a product a multiply-add (FP64 register operands)
+  FxTab fx;      // radius-1 stars: coefficients in canonical order, or centre and one for all others
 };
 
 // Element copy global -> shared through the asynchronous copy path (4, 8 or 16 bytes).
@@ -86,7 +89,37 @@ struct Tile4 {
 // vec: the input field's bricks start 16-byte aligned (16-byte copies allowed).
 constexpr int NT4 = 128;  // threads per CTA, each computing two of a brick's 256 points
 
-template <typename T, typename AT, int R, bool CANON>
+// Fixed point: the CTA's scan of a brick's values (the two centre values of each thread and four
+// values of the faces; a point's checked terms are its own and its i, j and k neighbours in the
+// lanes beside it, where point and neighbour differ in the lowest bit of the coordinate), from
+// every warp's through `slot`.  One block barrier.
+__device__ __forceinline__ FxScan fx_scan4(const double (&x)[6], const FxTab &tab, int2 *slot) {
+  FxScan s{0u, 0x7FFFFFFF};
+#pragma unroll
+  for (int q = 0; q < 6; ++q) s.top = max(s.top, fx_mag(x[q]));
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int a = (int)fx_mag(x[h]);
+    int m = a + tab.w[0];
+    m = __viaddmax_s32(__shfl_xor_sync(0xFFFFFFFFu, a, 1), tab.w[1], m);
+    m = __viaddmax_s32(__shfl_xor_sync(0xFFFFFFFFu, a, 4), tab.w[2], m);
+    m = __viaddmax_s32(__shfl_xor_sync(0xFFFFFFFFu, a, 16), tab.w[4], m);
+    s.term = min(s.term, m);
+  }
+  s.top = __reduce_max_sync(0xFFFFFFFFu, s.top);
+  s.term = __reduce_min_sync(0xFFFFFFFFu, s.term);
+  if ((threadIdx.x & 31) == 0) slot[threadIdx.x >> 5] = make_int2((int)s.top, s.term);
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < NT4 / 32; ++w) {
+    s.top = max(s.top, (unsigned)slot[w].x);
+    s.term = min(s.term, slot[w].y);
+  }
+  return s;
+}
+
+// FX: 0, or FxTab::on of a radius-1 star on FP64 storage.
+template <typename T, typename AT, int R, bool CANON, int FX>
 __global__ void __launch_bounds__(NT4)
 sweep4_kernel(const unsigned *__restrict__ adj, unsigned nbricks, const T *__restrict__ in, unsigned long long in_step,
               long long in_chunks, T *__restrict__ out, unsigned long long out_step, long long out_chunks,
@@ -254,6 +287,18 @@ sweep4_kernel(const unsigned *__restrict__ adj, unsigned nbricks, const T *__res
     if constexpr (F64) return fma(k, x, mz);
     else return k * x;
   };
+  // fixed point: the tile positions of this thread's face values, one per axis (threads 0 .. 63 the
+  // low faces, 64 .. 127 the high ones)
+  static_assert(FX == 0 || (F64 && CANON && R == 1), "fixed point: radius-1 stars on FP64 storage");
+  __shared__ int2 fxs[NT4 / 32];
+  int face[4];
+  if constexpr (FX != 0) {
+    const int x = t & 3, y = (t >> 2) & 3, z = (t >> 4) & 3, e = t < 64 ? -1 : B;
+    face[0] = G::toff(e + R, z + R, y + R, x) + C0;
+    face[1] = G::toff(z + R, e + R, y + R, x) + C0;
+    face[2] = G::toff(z + R, y + R, e + R, x) + C0;
+    face[3] = G::toff(z + R, y + R, x + R, e) + C0;
+  }
   int sc = 0, sb = 0;  // slot and buffer of brick jb (jb mod NSLOT, jb mod S)
   for (unsigned n = n0; n < nlist; n += gs) {
     const int sl = sc + S - 1 - (sc + S - 1 >= NSLOT ? NSLOT : 0);  // brick jb + S - 1
@@ -278,7 +323,48 @@ sweep4_kernel(const unsigned *__restrict__ adj, unsigned nbricks, const T *__res
     if (ob != NONE) {
       const T *c0 = tile[buf] + ctile[0], *c1 = tile[buf] + ctile[1];
       AT v0, v1;
-      if constexpr (CANON) {
+      bool done = false;
+      if constexpr (FX != 0) {
+        double x[6] = {c0[0], c1[0], tile[buf][face[0]], tile[buf][face[1]], tile[buf][face[2]], tile[buf][face[3]]};
+        const FxScan s = fx_scan4(x, tp.fx, fxs);
+        done = fx_ok(tp.fx, s);
+        if (done) {
+          constexpr int XB = FX == 2 ? 59 : 60;  // the sum of eight values stays below 2^62
+          const int E4 = (int)(s.top >> 20);
+          double *w = reinterpret_cast<double *>(tile[buf]);
+          const int at[6] = {ctile[0], ctile[1], face[0], face[1], face[2], face[3]};
+#pragma unroll
+          for (int q = 0; q < 6; ++q) {
+            const long long X = q < 2 ? fx_of_unit<XB>(x[q], E4) : fx_of<XB>(x[q], E4);
+            const int2 h = fx_split(X);
+            w[at[q]] = FX == 2 ? __longlong_as_double(X) : __hiloint2double(h.y, h.x);
+          }
+          __syncthreads();
+          const int scale = fx_scale<XB>(E4, tp.fx.q);
+          constexpr int O[8] = {-E * G::Q, E * G::Q, -G::Q, G::Q, -G::P, G::P, -1, 1};  // canonical order
+          auto point = [&](const T *c) -> double {
+            FxAcc<false> acc;
+            if constexpr (FX == 2) {
+              auto v = [&](int o) { return __double_as_longlong((double)c[o]); };
+              acc.first(tp.fx, 0, fx_split(v(0)));
+              long long y = v(O[0]) + v(O[1]) + v(O[2]);
+              y = y + v(O[3]) + v(O[4]);
+              y = y + v(O[5]) + v(O[6]);
+              acc.add(tp.fx, 1, fx_split(y + v(O[7])));
+            } else {
+              auto v = [&](int o) { return make_int2(__double2loint((double)c[o]), __double2hiint((double)c[o])); };
+              acc.first(tp.fx, 0, v(0));
+#pragma unroll
+              for (int q = 0; q < 8; ++q) acc.add(tp.fx, 1 + q, v(O[q]));
+            }
+            return fx_result(acc.sum(), scale);
+          };
+          v0 = (AT)point(c0);
+          v1 = (AT)point(c1);
+        }
+      }
+      if (done) {
+      } else if constexpr (CANON) {
         // the star of radius R in its canonical order: every tile offset a constant
         const AT k0 = F64 ? cr[0] : coefq(0);
         v0 = first(k0, c0[0]);
@@ -351,7 +437,19 @@ static int launch4(const unsigned *adj, unsigned nbricks, const bk_field *in, co
         tp.cf[q] = (float)c[q];
       }
   }
-  auto kern = canon ? sweep4_kernel<T, AT, R, true> : sweep4_kernel<T, AT, R, false>;
+  auto kern = canon ? sweep4_kernel<T, AT, R, true, 0> : sweep4_kernel<T, AT, R, false, 0>;
+  tp.fx.on = 0;
+  if constexpr (sizeof(T) == 8 && R == 1) {
+    // canonical order: centre, l -+, k -+, j -+, i -+; checked terms: centre, i, j and k
+    static const int near[5][9] = {{0, -1}, {7, 8, -1}, {5, 6, -1}, {0, -1}, {3, 4, -1}};
+    static const int first[9] = {0, 1, 2, 3, 4, 5, 6, 7, 8}, ones[9] = {1, 1, 1, 1, 1, 1, 1, 1, 1}, two[2] = {1, 8};
+    bool same = true;
+    for (int t = 2; t < MT && canon; ++t) same = same && tp.c[t] == tp.c[1];
+    if (canon && fx_table(tp.c, MT, near, 5, same ? 2 : 9, first, same ? two : ones, same ? 59 : 60, false, &tp.fx)) {
+      tp.fx.on = same ? 2 : 1;
+      kern = same ? sweep4_kernel<T, AT, R, true, 2> : sweep4_kernel<T, AT, R, true, 1>;
+    }
+  }
   const size_t smem = canon ? Tile4<T, R, true>::SMEM : G::SMEM;
   const char *ibase = reinterpret_cast<const char *>(in->dat) + in->offset * sizeof(T);
   const int vec = reinterpret_cast<uintptr_t>(ibase) % 16 == 0 && (in->step * sizeof(T)) % 16 == 0;

@@ -113,3 +113,51 @@ def test_fixed_point_short_lists_and_odd_output_fields(name, count, off):
     np.testing.assert_allclose(got[ids], full[ids], rtol=0, atol=3 * st.npoints * 2.0 ** -53 * float(np.abs(st.coeff).sum()))
     others = np.setdiff1d(np.arange(dom.nbricks), ids)
     assert not got[others].any()
+
+
+@pytest.mark.parametrize("kind", ["uniform", "same", "spread", "huge", "inf"])
+@pytest.mark.parametrize("ring", [True, False])
+def test_fixed_point_4d_stars_against_plain_sums(ring, kind):
+    """The radius-1 star on 4-D bricks: one coefficient for the eight neighbours (the values are
+    added before they are multiplied; `same`: all values just below a power of two, whose sum is the
+    largest there is), and nine different ones."""
+    from bricklib_gb300 import bricks4 as B4
+    lay, g = B4.Layout4(), (4, 3, 5, 4)
+    grid, adj = B4.init_grid(list(reversed(g)))
+    dims = tuple(4 * x for x in g)
+    arr = stencils.uniform(5, int(np.prod(dims))).reshape(dims)
+    rng = np.random.default_rng(2)
+    if kind == "same":
+        arr = np.full(dims, 1.0 - 2.0 ** -53)
+    elif kind == "spread":
+        arr = arr * 2.0 ** rng.integers(-40, 1, dims)
+    elif kind == "huge":
+        arr = arr * 1e299
+    elif kind == "inf":
+        arr[5, 5, 6, 7] = np.inf
+        arr[9, 6, 9, 5] = np.nan
+    st = B4.mpi9pt()
+    if not ring:
+        st.coeff = stencils.uniform(8, 9, 0.5, 1.0)
+    host = np.zeros(len(grid) * 512)
+    B4.copy_to_bricks(arr, grid, g, (0, 0, 0, 0), host, 512, 0, lay)
+    dev = B.movBrickStorage(B.BrickStorage(len(grid), 512, BK_F64, host=host))
+    a = B.DeviceBuffer(adj.nbytes)
+    a.upload(adj)
+    inner = grid.reshape(g)[1:-1, 1:-1, 1:-1, 1:-1]
+    B4.sweep4(a, len(grid), dev, 0, 256, B.BrickList(np.ascontiguousarray(inner.reshape(-1))), st, lay)
+    B.synchronize()
+    assert B.error_flags() == 0
+    out = B.movBrickStorage(dev, to_device=False).host
+    ig = tuple(x - 2 for x in g)
+    got = np.zeros(tuple(4 * x for x in ig))
+    B4.copy_from_bricks(got, inner, ig, (0, 0, 0, 0), out, 512, 256, lay)
+    want, size = np.zeros_like(got), np.zeros_like(got)
+    with np.errstate(all="ignore"):
+        for tap, c in zip(st.taps, st.coeff):
+            v = arr[tuple(slice(4 + o, 4 + o + n) for o, n in zip(tap, got.shape))]
+            want = want + c * v
+            size = size + np.abs(c * v)
+        fine = np.isfinite(want)
+        assert np.array_equal(fine, np.isfinite(got)) and np.array_equal(np.isnan(want), np.isnan(got))
+        assert (np.abs(got[fine] - want[fine]) <= 3 * 9 * 2.0 ** -53 * size[fine]).all()
