@@ -2,8 +2,10 @@
 // moves, the device error word, and the host-side periodic plan.
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "bk_common.cuh"
@@ -42,6 +44,36 @@ int *device_error_word() {
     g_err_words[dev] = p;
   }
   return g_err_words[dev];
+}
+
+int kernel_fit(const void *kern, int threads, size_t smem, int *sms, int *per_sm, const char *what) {
+  struct Fit {
+    int sms, per_sm;
+  };
+  static std::mutex mu;
+  static std::map<std::tuple<const void *, int, int, size_t>, Fit> fits;
+  static std::map<std::pair<const void *, int>, size_t> allowed;  // the attribute as last raised
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_fail(e, what);
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_tuple(kern, dev, threads, smem);
+  auto it = fits.find(key);
+  if (it == fits.end()) {
+    Fit f{0, 0};
+    e = cudaDeviceGetAttribute(&f.sms, cudaDevAttrMultiProcessorCount, dev);
+    size_t &most = allowed[{kern, dev}];
+    if (e == cudaSuccess && smem > 48 * 1024 && smem > most) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e == cudaSuccess) most = smem;
+    }
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f.per_sm, kern, threads, smem);
+    if (e != cudaSuccess) return cuda_fail(e, what);
+    it = fits.emplace(key, f).first;
+  }
+  *sms = it->second.sms;
+  *per_sm = it->second.per_sm;
+  return BK_OK;
 }
 
 int check_layout(const bk_layout *lay, Layout *out) {

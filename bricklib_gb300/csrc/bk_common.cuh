@@ -30,6 +30,12 @@ int *device_error_word();
 constexpr int FLAG_BOUNDS = 1;
 constexpr int FLAG_TIMEOUT = 2;
 
+// The CTAs of `threads` threads and `smem` bytes of dynamic shared memory that the current device
+// holds at a time: `sms` and resident CTAs per SM of a kernel.  Asked of the runtime once per
+// kernel, device and size (the queries took about as long as a launch); lets the kernel use that
+// much shared memory.
+int kernel_fit(const void *kern, int threads, size_t smem, int *sms, int *per_sm, const char *what);
+
 inline size_t dtype_size(int dt) { return dt == BK_F64 ? 8 : dt == BK_F32 ? 4 : 2; }
 inline bool dtype_ok(int dt) { return dt == BK_F64 || dt == BK_F32 || dt == BK_BF16; }
 
@@ -64,14 +70,9 @@ struct Layout {
     return vec * vl + lane;
   }
   __host__ __device__ __forceinline__ int size() const { return bk * bj * bi; }
-  // true when offset(k,j,i) == (k*bj + j)*bi + i for every element
-  __host__ bool row_major() const {
-    for (int k = 0; k < bk; ++k)
-      for (int j = 0; j < bj; ++j)
-        for (int i = 0; i < bi; ++i)
-          if (offset(k, j, i) != (k * bj + j) * bi + i) return false;
-    return true;
-  }
+  // true when offset(k,j,i) == (k*bj + j)*bi + i for every element: along i the fold spans the brick
+  // or is the only one with more than one element, along j likewise for what remains
+  __host__ bool row_major() const { return fi == bi ? fj == bj || fk == 1 : fj == 1 && fk == 1; }
 };
 
 int check_layout(const bk_layout *lay, Layout *out);

@@ -1560,13 +1560,9 @@ int launch_sweep2(const SweepArgs &a, const Taps &tp, cudaStream_t s, int grid_c
   static_assert(C::SMEM <= 227 * 1024, "tile too large");
   static_assert(BK * BJ * BI <= 8192 && C::TILE <= 16384, "plan entry fields overflow");
   auto kern = sweep2_kernel<T, BK, BJ, BI, R, FAM, ACC, BATCH, IST>;
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess && C::SMEM > 48 * 1024)
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, C::SMEM);
-  if (e != cudaSuccess) return cuda_fail(e, "sweep2 launch setup");
+  int sms = 0, per_sm = 0;
+  const int st = kernel_fit(reinterpret_cast<const void *>(kern), C::NT, C::SMEM, &sms, &per_sm, "sweep2 launch setup");
+  if (st) return st;
   if (per_sm < 1) return fail(BK_ERR_UNSUPPORTED, "sweep2 kernel does not fit on an SM");
   const long long groups = ((long long)a.nlist + C::NB - 1) / C::NB;
   long long grid = (long long)sms * per_sm;
@@ -1574,7 +1570,7 @@ int launch_sweep2(const SweepArgs &a, const Taps &tp, cudaStream_t s, int grid_c
   if (grid > groups) grid = groups;
   if (grid < 1) grid = 1;
   kern<<<(unsigned)grid, C::NT, C::SMEM, s>>>(a, tp);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "sweep2 kernel launch");
   return BK_OK;
 }

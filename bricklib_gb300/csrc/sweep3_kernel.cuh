@@ -681,12 +681,9 @@ int launch_star_tma(const SweepArgs &a, const Taps &tp, int dtype, cudaStream_t 
   TmaMaps maps;
   if (!star_tma_maps(a, dtype, BK, BJ, BI, R, C::IW, &maps)) return fail(BK_ERR_UNSUPPORTED, "field not describable to the TMA unit");
   auto kern = sweep_star_tma_kernel<T, BK, BJ, BI, R, ACC, NI>;
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, smem);
-  if (e != cudaSuccess) return cuda_fail(e, "star TMA sweep launch setup");
+  int sms = 0, per_sm = 0;
+  const int st = kernel_fit(reinterpret_cast<const void *>(kern), C::NT, smem, &sms, &per_sm, "star TMA sweep launch setup");
+  if (st) return st;
   if (per_sm < 1) return fail(BK_ERR_UNSUPPORTED, "star TMA sweep does not fit on an SM");
   const long long groups = ((long long)a.nlist + C::NB - 1) / C::NB;
   long long grid = (long long)sms * per_sm;
@@ -694,7 +691,7 @@ int launch_star_tma(const SweepArgs &a, const Taps &tp, int dtype, cudaStream_t 
   if (grid > groups) grid = groups;
   if (grid < 1) grid = 1;
   kern<<<(unsigned)grid, C::NT, smem, s>>>(maps, a, tp, S);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "star TMA sweep launch");
   return BK_OK;
 }

@@ -455,12 +455,9 @@ static int launch4(const unsigned *adj, unsigned nbricks, const bk_field *in, co
   const int vec = reinterpret_cast<uintptr_t>(ibase) % 16 == 0 && (in->step * sizeof(T)) % 16 == 0;
   int *err = device_error_word();
   if (!err) return fail(BK_ERR_CUDA, "device error word unavailable");
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaError_t e0 = cudaGetDevice(&dev);
-  if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e0 == cudaSuccess && smem > 48 * 1024) e0 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e0 == cudaSuccess) e0 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT4, smem);
-  if (e0 != cudaSuccess) return cuda_fail(e0, "sweep4 launch setup");
+  int sms = 0, per_sm = 0;
+  const int st = kernel_fit(reinterpret_cast<const void *>(kern), NT4, smem, &sms, &per_sm, "sweep4 launch setup");
+  if (st) return st;
   long long grid = (long long)sms * (per_sm > 0 ? per_sm : 1);
   if (grid > nlist) grid = nlist;
   if (grid < 1) grid = 1;

@@ -394,19 +394,16 @@ int launch_star_row(const SweepArgs &a, const Taps &tp, int dtype, cudaStream_t 
   static_assert((C::NB + 2) % SLOT_BOX == 0, "slot copies");
   const int group_maps = group && row_group_maps(a, dtype, C::BK, C::BJ, C::BI, R, C::NB, SLOT_BOX, &maps);
   auto kern = sweep_star_row_kernel<T, R, ACC>;
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, smem);
-  if (e != cudaSuccess) return cuda_fail(e, "row TMA sweep launch setup");
+  int sms = 0, per_sm = 0;
+  const int st = kernel_fit(reinterpret_cast<const void *>(kern), C::NT, smem, &sms, &per_sm, "row TMA sweep launch setup");
+  if (st) return st;
   if (per_sm < 1) return fail(BK_ERR_UNSUPPORTED, "row TMA sweep does not fit on an SM");
   const long long segs = ((long long)a.nlist + C::NB - 1) / C::NB;
   long long grid = (long long)sms * per_sm;
   if (grid > segs) grid = segs;
   if (grid < 1) grid = 1;
   kern<<<(unsigned)grid, C::NT, smem, s>>>(maps, a, tp, S, group_maps);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "row TMA sweep launch");
   return BK_OK;
 }
