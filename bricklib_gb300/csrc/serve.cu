@@ -7,9 +7,11 @@
 //              admission stream, its input is copied in and scattered into bricks there,
 //              and the tick stream waits on that before the job's first step;
 //   ticks      every active job advances one step per tick: one persistent sweep launch per
-//              (storage type, stencil) group over a work list of all active jobs' bricks.
-//              Jobs join and leave between ticks, so work of jobs that arrived at different
-//              times overlaps;
+//              (storage type, stencil) group over a work list of the group's jobs' bricks.  The
+//              groups share no data, so each runs its ticks on a stream of its own (lanes), and a
+//              group of few bricks does not leave the GPU idle while it runs; the lanes meet
+//              only where the work lists change.  Jobs join and leave between ticks, so work of
+//              jobs that arrived at different times overlaps;
 //   retirement after its last step a job's newest field is gathered into an array and
 //              copied to the client's output on a retire stream; a host callback on that
 //              stream stamps the completion time, releases its budget and wakes waiters.
@@ -140,7 +142,12 @@ struct bk_server {
   std::vector<std::pair<int, std::pair<unsigned, unsigned>>> work_seg;  // group -> (offset, count)
   unsigned ndom = 0;
   int parity = 0;
-  std::deque<cudaEvent_t> inflight;
+  // lanes: group q of the tick program runs on lane q mod NLANE.  fork: the program's tables are on
+  // the device; tick_ev[t mod NTICK][lane]: the lane is through tick t (bits of tick_used: lanes in use)
+  static constexpr int NLANE = 8, NTICK = 4;
+  cudaStream_t lanes[NLANE] = {};
+  cudaEvent_t fork = nullptr, join[NLANE] = {}, tick_ev[NTICK][NLANE] = {};
+  unsigned tick_used[NTICK] = {}, lanes_used = 0;  // lanes_used: lanes with ticks since the last fork
   // pinned staging for table uploads
   std::vector<unsigned char *> ring;
   std::vector<cudaEvent_t> ring_ev;
@@ -235,6 +242,13 @@ static int admit(bk_server *S, const std::shared_ptr<Job> &j) {
   return BK_OK;
 }
 
+// Lane of a group in the current tick program.
+static int lane_of(const bk_server *S, int group) {
+  for (size_t q = 0; q < S->work_seg.size(); ++q)
+    if (S->work_seg[q].first == group) return (int)(q % bk_server::NLANE);
+  return 0;
+}
+
 static int retire(bk_server *S, const std::shared_ptr<Job> &j, cudaEvent_t after_tick) {
   cudaStream_t s = S->s_retire;
   BK_CUDA(cudaStreamWaitEvent(s, after_tick, 0));
@@ -286,9 +300,16 @@ static unsigned char *ring_slot(bk_server *S, size_t bytes, int *slot) {
   return S->ring[r];
 }
 
-// rebuild the domain table and work list of the active jobs
+// rebuild the domain table and work list of the active jobs: on the tick stream, after every lane's
+// ticks of the program before (which read the tables freed here), before their next ones
 static int rebuild(bk_server *S) {
   cudaStream_t s = S->s_tick;
+  for (int l = 0; l < bk_server::NLANE; ++l)
+    if ((S->lanes_used >> l) & 1u) {
+      BK_CUDA(cudaEventRecord(S->join[l], S->lanes[l]));
+      BK_CUDA(cudaStreamWaitEvent(s, S->join[l], 0));
+    }
+  S->lanes_used = 0;
   std::vector<std::shared_ptr<Job>> order = S->active;
   std::stable_sort(order.begin(), order.end(), [](const std::shared_ptr<Job> &a, const std::shared_ptr<Job> &b) {
     return a->group < b->group;
@@ -335,19 +356,29 @@ static int rebuild(bk_server *S) {
   BK_CUDA(cudaEventRecord(S->ring_ev[slot], s));
   expand_work_kernel<<<n, 256, 0, s>>>(S->d_rows, n, S->d_work);
   BK_CUDA(cudaGetLastError());
+  BK_CUDA(cudaEventRecord(S->fork, s));
+  for (int l = 0; l < bk_server::NLANE; ++l) BK_CUDA(cudaStreamWaitEvent(S->lanes[l], S->fork, 0));
   S->active = order;
   return BK_OK;
 }
 
 static int tick(bk_server *S) {
-  cudaStream_t s = S->s_tick;
+  const int slot = (int)(S->ticks % bk_server::NTICK);
+  unsigned used = 0;
+  int q = 0;
   for (auto &ws : S->work_seg) {
     const Group &g = S->groups[ws.first];
+    const int l = q++ % bk_server::NLANE;
     // job storages come from cudaMallocAsync and hold two whole-brick fields: aligned
     int st = batch_launch_sweep(g.bs, g.dtype, S->d_doms, S->ndom, S->d_work + ws.second.first, ws.second.second,
-                                S->parity, S->L, S->err, 0, true, s);
+                                S->parity, S->L, S->err, 0, true, S->lanes[l]);
     if (st) return st;
+    used |= 1u << l;
   }
+  for (int l = 0; l < bk_server::NLANE; ++l)
+    if ((used >> l) & 1u) BK_CUDA(cudaEventRecord(S->tick_ev[slot][l], S->lanes[l]));
+  S->tick_used[slot] = used;
+  S->lanes_used |= used;
   S->parity ^= 1;
   S->ticks++;
   return BK_OK;
@@ -355,7 +386,6 @@ static int tick(bk_server *S) {
 
 static void serve_loop(bk_server *S) {
   cudaSetDevice(S->device);
-  const int MAXQ = 3;
   while (!S->stop) {
     // admission
     std::vector<std::shared_ptr<Job>> admitted;
@@ -400,14 +430,15 @@ static void serve_loop(bk_server *S) {
       }
       S->dirty = false;
     }
+    // bounded run-ahead of the host: the tick whose events this one takes over is through
+    const int slot = (int)(S->ticks % bk_server::NTICK);
+    for (int l = 0; l < bk_server::NLANE; ++l)
+      if ((S->tick_used[slot] >> l) & 1u) cudaEventSynchronize(S->tick_ev[slot][l]);
     int st = tick(S);
     if (st != BK_OK) {
       S->fatal = bk_last_error();
       break;
     }
-    cudaEvent_t ev = nullptr;
-    cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-    cudaEventRecord(ev, S->s_tick);
     // retire finished jobs
     std::vector<std::shared_ptr<Job>> still;
     for (auto &j : S->active) {
@@ -415,7 +446,7 @@ static void serve_loop(bk_server *S) {
         still.push_back(j);
         continue;
       }
-      if (retire(S, j, ev) != BK_OK) {
+      if (retire(S, j, S->tick_ev[slot][lane_of(S, j->group)]) != BK_OK) {
         std::lock_guard<std::mutex> lk(S->mu);
         j->error = bk_last_error();
         j->state = JOB_FAILED;
@@ -424,12 +455,6 @@ static void serve_loop(bk_server *S) {
       S->dirty = true;
     }
     S->active.swap(still);
-    S->inflight.push_back(ev);
-    while ((int)S->inflight.size() > MAXQ) {  // bounded run-ahead of the host
-      cudaEventSynchronize(S->inflight.front());
-      cudaEventDestroy(S->inflight.front());
-      S->inflight.pop_front();
-    }
   }
   {
     std::lock_guard<std::mutex> lk(S->mu);
@@ -457,6 +482,13 @@ int bk_server_create(bk_server **out, size_t hbm_budget, const bk_layout *lay, i
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&S->s_tick, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&S->s_admit, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&S->s_retire, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&S->fork, cudaEventDisableTiming);
+  for (int l = 0; l < bk_server::NLANE && e == cudaSuccess; ++l) {
+    e = cudaStreamCreateWithFlags(&S->lanes[l], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&S->join[l], cudaEventDisableTiming);
+    for (int t = 0; t < bk_server::NTICK && e == cudaSuccess; ++t)
+      e = cudaEventCreateWithFlags(&S->tick_ev[t][l], cudaEventDisableTiming);
+  }
   if (e == cudaSuccess) {
     // keep freed blocks in the stream-ordered pool instead of returning them to the driver
     cudaMemPool_t pool;
@@ -597,7 +629,12 @@ int bk_server_destroy(bk_server *S) {
     if (j.grid) cudaFree(j.grid);
     if (j.ready) cudaEventDestroy(j.ready);
   }
-  for (auto ev : S->inflight) cudaEventDestroy(ev);
+  for (int l = 0; l < bk_server::NLANE; ++l) {
+    cudaStreamDestroy(S->lanes[l]);
+    cudaEventDestroy(S->join[l]);
+    for (int t = 0; t < bk_server::NTICK; ++t) cudaEventDestroy(S->tick_ev[t][l]);
+  }
+  cudaEventDestroy(S->fork);
   if (S->d_doms) cudaFree(S->d_doms);
   if (S->d_work) cudaFree(S->d_work);
   if (S->d_rows) cudaFree(S->d_rows);
