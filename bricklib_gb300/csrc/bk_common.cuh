@@ -30,6 +30,28 @@ int *device_error_word();
 constexpr int FLAG_BOUNDS = 1;
 constexpr int FLAG_TIMEOUT = 2;
 
+// Launch of a kernel that begins with grid_begin(): it is brought up, as far as it needs no global
+// memory, while the stream's previous kernel ends (programmatic dependent launch).  Sweeps in a row,
+// us each, without / with it: 7-point Laplacian 128^3 32.0 / 29.8, heat step 128^3 15.9 / 13.7 and 256^3
+// 77.2 / 74.8.  Inside a stream capture, where the previous node need not be a kernel, an ordinary
+// launch.
+template <class... P, class... A>
+cudaError_t launch_overlapped(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, const A &...args) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool eager = cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = eager ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // The CTAs of `threads` threads and `smem` bytes of dynamic shared memory that the current device
 // holds at a time: `sms` and resident CTAs per SM of a kernel.  Asked of the runtime once per
 // kernel, device and size (the queries took about as long as a launch); lets the kernel use that
@@ -40,6 +62,13 @@ inline size_t dtype_size(int dt) { return dt == BK_F64 ? 8 : dt == BK_F32 ? 4 : 
 inline bool dtype_ok(int dt) { return dt == BK_F64 || dt == BK_F32 || dt == BK_BF16; }
 
 // ---------------------------------------------------------------- element types
+
+// First in a kernel, before any access to global memory: waits until the stream's previous kernel is
+// through and its writes are visible.  Every thread calls it, so a grid never ends before the one it
+// waits for.  (No early trigger, griddepcontrol.launch_dependents: with it the next grid's CTAs
+// took the places of the first ones to end and the 7-point Laplacian at 128^3 went from 29.8 to
+// 32.7 us a sweep, the 125-point cube at 512^3 from 2272 to 2329.)
+__device__ __forceinline__ void grid_begin() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 template <typename T> struct Elem;
 template <> struct Elem<double> {

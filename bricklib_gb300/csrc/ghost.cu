@@ -12,6 +12,7 @@ __global__ void __launch_bounds__(256)
 ghost_fill_kernel(const unsigned *__restrict__ pairs, unsigned npairs, unsigned char *dat,
                   unsigned long long step_bytes, unsigned long long off_bytes, unsigned words,
                   long long chunks, int *err) {
+  grid_begin();
   if (words <= blockDim.x) {
     const unsigned t = threadIdx.x;
     for (unsigned p0 = blockIdx.x * GF_PAIRS; p0 < npairs; p0 += gridDim.x * GF_PAIRS) {
@@ -89,13 +90,13 @@ int ghost_fill(const unsigned *pairs, unsigned npairs, const bk_field *f, const 
   const unsigned groups = (npairs + GF_PAIRS - 1) / GF_PAIRS;
   const unsigned grid = groups < (1u << 30) ? groups : (1u << 30);
   unsigned char *dat = reinterpret_cast<unsigned char *>(f->dat);
+  cudaError_t e = cudaSuccess;
   if (((base | step_b | off_b | bytes) & 15) == 0)
-    ghost_fill_kernel<uint4><<<grid, 256, 0, s>>>(pairs, npairs, dat, step_b, off_b, (unsigned)(bytes / 16), f->chunks, err);
+    e = launch_overlapped(ghost_fill_kernel<uint4>, grid, 256, 0, s, pairs, npairs, dat, step_b, off_b, (unsigned)(bytes / 16), f->chunks, err);
   else if (((base | step_b | off_b | bytes) & 7) == 0)
-    ghost_fill_kernel<uint2><<<grid, 256, 0, s>>>(pairs, npairs, dat, step_b, off_b, (unsigned)(bytes / 8), f->chunks, err);
+    e = launch_overlapped(ghost_fill_kernel<uint2>, grid, 256, 0, s, pairs, npairs, dat, step_b, off_b, (unsigned)(bytes / 8), f->chunks, err);
   else
-    ghost_fill_kernel<unsigned short><<<grid, 256, 0, s>>>(pairs, npairs, dat, step_b, off_b, (unsigned)(bytes / 2), f->chunks, err);
-  cudaError_t e = cudaGetLastError();
+    e = launch_overlapped(ghost_fill_kernel<unsigned short>, grid, 256, 0, s, pairs, npairs, dat, step_b, off_b, (unsigned)(bytes / 2), f->chunks, err);
   if (e != cudaSuccess) return cuda_fail(e, "ghost fill launch");
   return BK_OK;
 }

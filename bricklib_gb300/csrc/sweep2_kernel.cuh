@@ -1476,6 +1476,7 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
   static_assert(!C::FX || (TPB == 64 && BK == 8 && BJ == 8 && BI == 8 && (FAM == FAM_STAR || FAM == FAM_CUBE)),
                 "fixed point: stars and cubes on 8x8x8 bricks, 64 threads each");
 
+  grid_begin();
   // prologue: adjacency of the first two groups, copies of the first
   Walk w1{g0, 0};
   Walk w2 = advance(w1), w3 = advance(w2);  // the next group and the one after
@@ -1569,8 +1570,13 @@ int launch_sweep2(const SweepArgs &a, const Taps &tp, cudaStream_t s, int grid_c
   if (grid_cap > 0 && grid > grid_cap) grid = grid_cap;
   if (grid > groups) grid = groups;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, C::NT, C::SMEM, s>>>(a, tp);
-  const cudaError_t e = cudaGetLastError();
+  cudaError_t e = cudaSuccess;
+  if constexpr (BATCH) {  // the server's lanes: CTAs that wait for one lane would hold room others need
+    kern<<<(unsigned)grid, C::NT, C::SMEM, s>>>(a, tp);
+    e = cudaGetLastError();
+  } else {
+    e = launch_overlapped(kern, (unsigned)grid, C::NT, C::SMEM, s, a, tp);
+  }
   if (e != cudaSuccess) return cuda_fail(e, "sweep2 kernel launch");
   return BK_OK;
 }

@@ -481,6 +481,7 @@ sweep_star_tma_kernel(const __grid_constant__ TmaMaps maps, const SweepArgs a, c
   if (threadIdx.x < F64Ops::NHEAD + C::NTAP)
     coef_s[threadIdx.x] = threadIdx.x < F64Ops::NHEAD ? tp.one_mz[threadIdx.x] : tp.c[threadIdx.x - F64Ops::NHEAD];
   __syncthreads();
+  grid_begin();
 
   const long long ngroups = ((long long)a.nlist + NB - 1) / NB;
   const long long g0 = blockIdx.x, gstep = gridDim.x;
@@ -690,8 +691,7 @@ int launch_star_tma(const SweepArgs &a, const Taps &tp, int dtype, cudaStream_t 
   if (grid_cap > 0 && grid > grid_cap) grid = grid_cap;
   if (grid > groups) grid = groups;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, C::NT, smem, s>>>(maps, a, tp, S);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_overlapped(kern, (unsigned)grid, C::NT, smem, s, maps, a, tp, S);
   if (e != cudaSuccess) return cuda_fail(e, "star TMA sweep launch");
   return BK_OK;
 }

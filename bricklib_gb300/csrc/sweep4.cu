@@ -190,6 +190,7 @@ sweep4_kernel(const unsigned *__restrict__ adj, unsigned nbricks, const T *__res
     nneed = c;
   }
   __syncthreads();
+  grid_begin();
   // list positions in 32 bits: the host holds lists below 2^31 entries, so n + (S + 3) gs stays
   // far below 2^32
   const unsigned gs = gridDim.x;
@@ -461,10 +462,9 @@ static int launch4(const unsigned *adj, unsigned nbricks, const bk_field *in, co
   long long grid = (long long)sms * (per_sm > 0 ? per_sm : 1);
   if (grid > nlist) grid = nlist;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, NT4, smem, s>>>(
-      adj, nbricks, reinterpret_cast<const T *>(in->dat) + in->offset, in->step, in->chunks,
-      reinterpret_cast<T *>(out->dat) + out->offset, out->step, out->chunks, blist, nlist, L, tp, star, vec, err);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_overlapped(
+      kern, (unsigned)grid, NT4, smem, s, adj, nbricks, reinterpret_cast<const T *>(in->dat) + in->offset, in->step,
+      in->chunks, reinterpret_cast<T *>(out->dat) + out->offset, out->step, out->chunks, blist, nlist, L, tp, star, vec, err);
   if (e != cudaSuccess) return cuda_fail(e, "sweep4 launch");
   return BK_OK;
 }

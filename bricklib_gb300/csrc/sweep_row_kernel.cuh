@@ -171,6 +171,7 @@ sweep_star_row_kernel(const __grid_constant__ TmaMaps maps, const SweepArgs a, c
     fence_proxy_async_smem();
   }
   __syncthreads();
+  grid_begin();
 
   const long long nseg = ((long long)a.nlist + NB - 1) / NB;
   const long long g0 = blockIdx.x, gstep = gridDim.x;
@@ -402,8 +403,7 @@ int launch_star_row(const SweepArgs &a, const Taps &tp, int dtype, cudaStream_t 
   long long grid = (long long)sms * per_sm;
   if (grid > segs) grid = segs;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, C::NT, smem, s>>>(maps, a, tp, S, group_maps);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_overlapped(kern, (unsigned)grid, C::NT, smem, s, maps, a, tp, S, group_maps);
   if (e != cudaSuccess) return cuda_fail(e, "row TMA sweep launch");
   return BK_OK;
 }
