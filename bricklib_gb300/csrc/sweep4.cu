@@ -89,10 +89,10 @@ struct Tile4 {
 // vec: the input field's bricks start 16-byte aligned (16-byte copies allowed).
 constexpr int NT4 = 128;  // threads per CTA, each computing two of a brick's 256 points
 
-// Fixed point: the CTA's scan of a brick's values (the two centre values of each thread and four
-// values of the faces; a point's checked terms are its own and its i, j and k neighbours in the
-// lanes beside it, where point and neighbour differ in the lowest bit of the coordinate), from
-// every warp's through `slot`.  One block barrier.
+// Fixed point: the CTA's scan of a brick's values (the two centre values of each thread, neighbours
+// along l, and four values of the faces; a point's checked terms are its own, its l neighbour in
+// the thread and its i neighbour in the lane beside it), from every warp's through `slot`.  One
+// block barrier.
 __device__ __forceinline__ FxScan fx_scan4(const double (&x)[6], const FxTab &tab, int2 *slot) {
   FxScan s{0u, 0x7FFFFFFF};
 #pragma unroll
@@ -102,8 +102,7 @@ __device__ __forceinline__ FxScan fx_scan4(const double (&x)[6], const FxTab &ta
     const int a = (int)fx_mag(x[h]);
     int m = a + tab.w[0];
     m = __viaddmax_s32(__shfl_xor_sync(0xFFFFFFFFu, a, 1), tab.w[1], m);
-    m = __viaddmax_s32(__shfl_xor_sync(0xFFFFFFFFu, a, 4), tab.w[2], m);
-    m = __viaddmax_s32(__shfl_xor_sync(0xFFFFFFFFu, a, 16), tab.w[4], m);
+    m = __viaddmax_s32((int)fx_mag(x[h ^ 1]), tab.w[2], m);
     s.term = min(s.term, m);
   }
   s.top = __reduce_max_sync(0xFFFFFFFFu, s.top);
@@ -259,13 +258,15 @@ sweep4_kernel(const unsigned *__restrict__ adj, unsigned nbricks, const T *__res
   __syncthreads();  // the first S adjacency slots
 #pragma unroll
   for (int q = 0; q + 1 < S; ++q) issue(q, q);
-  // this thread's output elements t and t + NT4: their tile positions and in-brick offsets
+  // this thread's two output elements, neighbours along l: their tile positions and in-brick offsets
   static_assert(2 * NT4 == B * B * B * B, "two points per thread");
   int ctile[2], oofs[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    const int pt = t + NT4 * h;
-    const int oi = pt % B, oj = (pt / B) % B, ok = (pt / (B * B)) % B, ol = pt / (B * B * B);
+    // FP64: k before j, since four k planes' rows (Q = 36 elements apart) fall in different banks and
+    // four j rows (6 apart) do not
+    const int oi = t % B, o1 = (t / B) % B, o2 = (t / (B * B)) % B, ol = 2 * (t / (B * B * B)) + h;
+    const int oj = G::ES == 8 ? o2 : o1, ok = G::ES == 8 ? o1 : o2;
     ctile[h] = G::toff(ol + R, ok + R, oj + R, oi) + C0;
     oofs[h] = L.offset(ol, ok, oj, oi);
   }
@@ -295,7 +296,7 @@ sweep4_kernel(const unsigned *__restrict__ adj, unsigned nbricks, const T *__res
   int face[4];
   if constexpr (FX != 0) {
     const int x = t & 3, y = (t >> 2) & 3, z = (t >> 4) & 3, e = t < 64 ? -1 : B;
-    face[0] = G::toff(e + R, z + R, y + R, x) + C0;
+    face[0] = G::toff(e + R, y + R, z + R, x) + C0;
     face[1] = G::toff(z + R, e + R, y + R, x) + C0;
     face[2] = G::toff(z + R, y + R, e + R, x) + C0;
     face[3] = G::toff(z + R, y + R, x + R, e) + C0;
@@ -334,34 +335,39 @@ sweep4_kernel(const unsigned *__restrict__ adj, unsigned nbricks, const T *__res
           const int E4 = (int)(s.top >> 20);
           double *w = reinterpret_cast<double *>(tile[buf]);
           const int at[6] = {ctile[0], ctile[1], face[0], face[1], face[2], face[3]};
+          double v[6];
 #pragma unroll
           for (int q = 0; q < 6; ++q) {
             const long long X = q < 2 ? fx_of_unit<XB>(x[q], E4) : fx_of<XB>(x[q], E4);
             const int2 h = fx_split(X);
-            w[at[q]] = FX == 2 ? __longlong_as_double(X) : __hiloint2double(h.y, h.x);
+            v[q] = FX == 2 ? __longlong_as_double(X) : __hiloint2double(h.y, h.x);
+            w[at[q]] = v[q];
           }
           __syncthreads();
           const int scale = fx_scale<XB>(E4, tp.fx.q);
           constexpr int O[8] = {-E * G::Q, E * G::Q, -G::Q, G::Q, -G::P, G::P, -1, 1};  // canonical order
-          auto point = [&](const T *c) -> double {
+          auto point = [&](const T *c, int h) -> double {  // the thread's own two values from registers
+            double n[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) n[q] = q == 1 - h ? v[1 - h] : (double)c[O[q]];
             FxAcc<false> acc;
             if constexpr (FX == 2) {
-              auto v = [&](int o) { return __double_as_longlong((double)c[o]); };
-              acc.first(tp.fx, 0, fx_split(v(0)));
-              long long y = v(O[0]) + v(O[1]) + v(O[2]);
-              y = y + v(O[3]) + v(O[4]);
-              y = y + v(O[5]) + v(O[6]);
-              acc.add(tp.fx, 1, fx_split(y + v(O[7])));
+              auto ll = [](double d) { return __double_as_longlong(d); };
+              acc.first(tp.fx, 0, fx_split(ll(v[h])));
+              long long y = ll(n[0]) + ll(n[1]) + ll(n[2]);
+              y = y + ll(n[3]) + ll(n[4]);
+              y = y + ll(n[5]) + ll(n[6]);
+              acc.add(tp.fx, 1, fx_split(y + ll(n[7])));
             } else {
-              auto v = [&](int o) { return make_int2(__double2loint((double)c[o]), __double2hiint((double)c[o])); };
-              acc.first(tp.fx, 0, v(0));
+              auto half = [](double d) { return make_int2(__double2loint(d), __double2hiint(d)); };
+              acc.first(tp.fx, 0, half(v[h]));
 #pragma unroll
-              for (int q = 0; q < 8; ++q) acc.add(tp.fx, 1 + q, v(O[q]));
+              for (int q = 0; q < 8; ++q) acc.add(tp.fx, 1 + q, half(n[q]));
             }
             return fx_result(acc.sum(), scale);
           };
-          v0 = (AT)point(c0);
-          v1 = (AT)point(c1);
+          v0 = (AT)point(c0, 0);
+          v1 = (AT)point(c1, 1);
         }
       }
       if (done) {
@@ -441,12 +447,12 @@ static int launch4(const unsigned *adj, unsigned nbricks, const bk_field *in, co
   auto kern = canon ? sweep4_kernel<T, AT, R, true, 0> : sweep4_kernel<T, AT, R, false, 0>;
   tp.fx.on = 0;
   if constexpr (sizeof(T) == 8 && R == 1) {
-    // canonical order: centre, l -+, k -+, j -+, i -+; checked terms: centre, i, j and k
-    static const int near[5][9] = {{0, -1}, {7, 8, -1}, {5, 6, -1}, {0, -1}, {3, 4, -1}};
+    // canonical order: centre, l -+, k -+, j -+, i -+; checked terms: centre, i and l
+    static const int near[3][9] = {{0, -1}, {7, 8, -1}, {1, 2, -1}};
     static const int first[9] = {0, 1, 2, 3, 4, 5, 6, 7, 8}, ones[9] = {1, 1, 1, 1, 1, 1, 1, 1, 1}, two[2] = {1, 8};
     bool same = true;
     for (int t = 2; t < MT && canon; ++t) same = same && tp.c[t] == tp.c[1];
-    if (canon && fx_table(tp.c, MT, near, 5, same ? 2 : 9, first, same ? two : ones, same ? 59 : 60, false, &tp.fx)) {
+    if (canon && fx_table(tp.c, MT, near, 3, same ? 2 : 9, first, same ? two : ones, same ? 59 : 60, false, &tp.fx)) {
       tp.fx.on = same ? 2 : 1;
       kern = same ? sweep4_kernel<T, AT, R, true, 2> : sweep4_kernel<T, AT, R, true, 1>;
     }
