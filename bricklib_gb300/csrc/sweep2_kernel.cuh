@@ -171,14 +171,18 @@ struct Sweep2Cfg {
   // (two-way within a half warp, which reads half the bytes of the FP32 case)
   static constexpr bool CS4 = IST && ES <= 4;
   static constexpr bool SWZ = BK_CS_SWZ && CS4 && ES == 4 && BI + 2 * RP == 16;
-  static constexpr int EI = CS4 ? (ES == 4 ? (SWZ ? 16 : 20) : 24)
+  // the FP32 27-point cube on column pairs: rows of 12, the one halo value of either side by a 4-byte
+  // copy (low: before the centre; high: at the next row's front, unused there), half the tile of
+  // rows held as whole 16-byte copies and padded to 24: twice the resident CTAs
+  static constexpr bool HALO4 = ES == 4 && FAM == FAM_CUBE && R == 1 && BK == 8 && BJ == 8 && BI == 8 && ACC == ACCM_NATIVE;
+  static constexpr int EI = HALO4 ? BI + RP : CS4 ? (ES == 4 ? (SWZ ? 16 : 20) : 24)
                           : PERM ? (NEED % 8 <= 4 ? NEED - NEED % 8 + 4 : NEED - NEED % 8 + 12)
                                  : conflict_free_row(NEED, BI, ES, VE);
   // the 125-point cube in fixed point: planes two elements longer, so that a quarter warp's pair loads
   // from four rows of two planes fall in different banks
   static constexpr bool FX125 = FAM == FAM_CUBE && R == 2 && ACC == ACCM_FXS;
   static constexpr int SK = EJ * EI + (FX125 ? 2 : 0);  // elements per plane
-  static constexpr int TILE = EK * SK;                  // elements per brick tile
+  static constexpr int TILE = EK * SK + (HALO4 ? VE : 0);  // elements per brick tile
   // position within tile row jj of column ii (SWZ: the row's 16-byte units permuted)
   static __host__ __device__ __forceinline__ int col(int jj, int ii) {
     return SWZ ? ((((ii >> 2) ^ ((jj >> 1) & 3)) << 2) | (ii & 3)) : ii;
@@ -203,7 +207,8 @@ struct Sweep2Cfg {
   static constexpr int NV_JF = BK * R * (BI / VE);   // one j face
   static constexpr int NV_IF = BK * BJ * (RP / VE);  // one i face
   static constexpr int NV_STAR = NV_CENTRE + 2 * (NV_KF + NV_JF + NV_IF);
-  static constexpr int NV_CUBE = EK * EJ * (NEED / VE);  // the row padding is never fetched
+  static constexpr int NV_ROWS = EK * EJ * (BI / VE);  // HALO4: the centre rows, then two halo values a row
+  static constexpr int NV_CUBE = HALO4 ? NV_ROWS + 2 * EK * EJ : EK * EJ * (NEED / VE);  // the row padding is never fetched
   static constexpr int NV = FAM == FAM_STAR ? NV_STAR : NV_CUBE;
   static constexpr int EPT = (NV + TPB - 1) / TPB;  // plan entries per thread
   // float-float converts each raw FP64 tile into float pairs in place (same 8 bytes)
@@ -237,6 +242,14 @@ struct Sweep2Cfg {
 template <typename C, int BK, int BJ, int BI, int R, int FAM>
 __device__ __forceinline__ void plan_coords(int g, int &kk, int &jj, int &ii) {
   constexpr int VE = C::VE, RP = C::RP;
+  if constexpr (C::HALO4) {
+    const bool halo = g >= C::NV_ROWS;
+    const int h = g - C::NV_ROWS, row = halo ? h >> 1 : g / (BI / VE);
+    kk = row / C::EJ;
+    jj = row % C::EJ;
+    ii = halo ? ((h & 1) ? RP + BI : RP - 1) : RP + (g % (BI / VE)) * VE;
+    return;
+  }
   if (FAM != FAM_STAR) {
     constexpr int RV = C::NEED / VE;
     kk = g / (C::EJ * RV);
@@ -893,7 +906,8 @@ __device__ __forceinline__ void sweep2_brick(const T *rt, T *out_brick, int lt, 
   if constexpr (C::PAIR) {
     // lane -> (row, column pair); 16-byte pairs: rows 0,2,1,3 per quarter warp, two rows apart
     const int q = lt >> 2, i0 = 2 * (lt & 3);
-    const int jp = C::PERM ? (q & 4) | ((q & 1) << 1) | ((q >> 1) & 1) : q;
+    // (rows of 12 words: the even rows' pairs fall in different banks, and the odd rows')
+    const int jp = C::PERM ? (q & 4) | ((q & 1) << 1) | ((q >> 1) & 1) : C::HALO4 ? ((q & 3) << 1) | (q >> 2) : q;
     if constexpr (C::ES == 8)
       sym_cube_pair_shared<C, T, R, FAM == FAM_CUBESYM_IJ>(rt, out_brick + (size_t)(jp * BI + i0), jp, i0, tp);
     else
@@ -1454,7 +1468,8 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
         if (e < ne && need && p != 0xFFFFFFFFu) {
           const unsigned sl = p & 31u, src = (p >> 5) & 8191u, dst = p >> 18;
           const T *g = in + (size_t)nbr[sl] * step + src;
-          cp_async<C::VB>(tbase + dst * C::ES, g);
+          if (C::HALO4 && e * TPB + lt >= C::NV_ROWS) cp_async<4>(tbase + dst * C::ES, g);
+          else cp_async<C::VB>(tbase + dst * C::ES, g);
         }
       }
     }
