@@ -326,6 +326,44 @@ struct FxTile {
     return p < 2 ? pk + 10 * SK * p : p < 4 ? pj + 10 * SJ * (p - 2) : pi + 10 * (p - 4);
   }
   __device__ __forceinline__ int one(int p) const { return pi + 9 * p; }
+  // position of this thread's (j, i) column at plane k of its four (k in -R .. 3 + R), its warp w
+  __device__ __forceinline__ static void columns(int j, int i, int w, int (&c)[3]) {
+    c[0] = c[1] = c[2] = at(4 * w, j, i);
+  }
+};
+// Radius 4: planes 0 .. 7 of 16 rows (-4 .. 11) of 18 (columns -4 .. 11); the four corners of a plane,
+// which a star does not read, hold the quarters of a k-face plane: plane -4 + q in plane q, plane 8 + q
+// in plane 4 + q.  18 KB instead of 32 for the whole box.
+template <>
+struct FxTile<4> {
+  static constexpr int SJ = 18, SK = 16 * SJ, SIZE = 8 * SK;
+  static __device__ __forceinline__ int row(int lt) {
+    const int q = (lt >> 2) & 7;
+    return (q >> 1) | ((q & 1) << 2);
+  }
+  int pk, pj, pi;
+  static __device__ __forceinline__ int at(int k, int j, int i) { return k * SK + (j + 4) * SJ + i + 4; }
+  // row j or column i of a k-face plane, in the corners
+  static __device__ __forceinline__ int corner(int x) { return x < 4 ? x - 4 : x + 4; }
+  __device__ __forceinline__ FxTile(int lt) {
+    const int i = 2 * (lt & 3);
+    pk = at(lt >> 5, corner((lt >> 2) & 7), corner(i));
+    pj = at(lt >> 4, ((lt >> 2) & 3) - 4, i);
+    pi = at(lt >> 4, (lt >> 1) & 7, 2 * (lt & 1) - 4);
+  }
+  __device__ __forceinline__ int block(int k, int j, int i) const { return at(k, j, i); }
+  __device__ __forceinline__ bool has(int) const { return true; }
+  __device__ __forceinline__ int pair(int p) const {
+    return p < 4 ? pk + 2 * SK * p : p < 8 ? pj + 4 * SK * (p & 1) + (p >= 6 ? 12 * SJ : 0)
+                                           : pi + 4 * SK * (p & 1) + (p >= 10 ? 12 : 0);
+  }
+  __device__ __forceinline__ int one(int) const { return 0; }
+  __device__ __forceinline__ static void columns(int j, int i, int w, int (&c)[3]) {
+    const int centre = at(0, j, i), face = at(0, corner(j), corner(i));
+    c[0] = (w ? centre : face) + 4 * SK;  // planes -4 .. -1 of the thread
+    c[1] = centre + 4 * w * SK;           // 0 .. 3
+    c[2] = w ? face : centre;             // 4 .. 7
+  }
 };
 
 // Cubes: the (8 + 2R)^3 box without its centre, value n of the list to thread n mod 64; the

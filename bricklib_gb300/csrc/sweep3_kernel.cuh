@@ -63,9 +63,9 @@ struct StarTmaCfg {
   // ... and the fixed-point scans, [call parity][brick][warp] int2 (16-byte aligned)
   static constexpr int O_SCAN = (O_COEF + 8 * (F64Ops::NHEAD + NTAP) + 15) / 16 * 16;
   static constexpr int META = O_SCAN + 2 * NB * 2 * 8;
-  // fixed point of radius 1 and 2: a tile of integers per brick after the meta data (128-byte aligned)
+  // fixed point: a tile of integers per brick after the meta data (128-byte aligned)
   static constexpr int fx_tile(int acc) {
-    return R <= 2 && ES == 8 && (acc == ACCM_FX || acc == ACCM_FXS) ? FxTile<R <= 2 ? R : 1>::SIZE * 8 : 0;
+    return ES == 8 && (acc == ACCM_FX || acc == ACCM_FXS) ? FxTile<R>::SIZE * 8 : 0;
   }
   static constexpr int o_tile(int stages) { return (stages * NB * BRICK + META + 127) / 128 * 128; }
   static constexpr int smem(int stages, int acc) {  // + base alignment slack
@@ -341,31 +341,28 @@ __device__ __forceinline__ void star_column_f64_of(const double *buf, const int 
                               cs + F64Ops::NHEAD, F64Ops::load(cs));
 }
 
-// The consumer threads of a fixed-point star sweep (fx.cuh): 64 threads (two warps) per brick.
-// Radius 1 and 2: the values are read from the stage into registers, the stage goes back to the
-// producer, and the integers go to a tile of their own, where every tap is at a constant distance
-// (a stage's faces each have strides of their own) and the next brick's copies run meanwhile.
-// Radius 4, whose tile would take 32 KB: in the stage, in place.
+// The consumer threads of a fixed-point star sweep (fx.cuh): 64 threads (two warps) per brick.  The
+// values are read from the stage into registers, the stage goes back to the producer, and the
+// integers go to a tile of their own, where every tap is at a constant distance (a stage's faces
+// each have strides of their own) and the next brick's copies run meanwhile.
 template <typename C, int R, bool SUM>
 __device__ __forceinline__ void star_fx_consume(unsigned char *sm, const unsigned full0, const unsigned empty0,
                                                 const unsigned *outb, volatile int *abort_word, const int S,
                                                 const int bs, const int lt, const SweepArgs &a, const Taps &tp,
                                                 const long long ngroups, const unsigned long long lim) {
   constexpr int NB = C::NB, IW = C::IW;
-  constexpr bool TILE = R <= 2;
+  typedef FxTile<R> X;
   static_assert(C::TPB == 64 && NB <= 2 && C::ES == 8, "8x8x8 bricks of FP64");
   static_assert(C::O_KL == 4096 && C::BRICK == C::O_KL + 8 * (256 * R + 128 * IW), "faces one after the other");
   const int lane = lt & 31;
   int2 *scan = reinterpret_cast<int2 *>(sm + S * NB * C::BRICK + C::O_SCAN) + 2 * bs;
   double *tile = reinterpret_cast<double *>(sm + C::o_tile(S) + bs * C::fx_tile(ACCM_FX));
-  const auto share = [&] {
-    const FxDense<R, IW> dense{lt};
-    if constexpr (TILE) return fx_share<true, true, SUM, false, 60>(lt, dense, FxTile<R>(lt));
-    else return fx_share<true, true, SUM, false, 60>(lt, dense, dense);
-  }();
-  // this thread's column pair and four planes.  In the tile a quarter warp takes rows two apart
-  const int q8 = (lt >> 2) & 7, pi = 2 * (lt & 3), pk = 4 * (lt >> 5);
-  const int pj = TILE ? FxTile<TILE ? R : 1>::row(lt) : q8;
+  const auto share = fx_share<true, true, SUM, false, 60>(lt, FxDense<R, IW>{lt}, X(lt));
+  // this thread's column pair and four planes
+  const int pj = X::row(lt), pi = 2 * (lt & 3), pk = 4 * (lt >> 5);
+  int col[3];
+  X::columns(pj, pi, lt >> 5, col);
+  const double *c0 = tile + col[0], *c1 = tile + col[1], *c2 = tile + col[2];
   int st = 0;
   unsigned ph = 0;   // phase parity of the stage's current use
   unsigned par = 0;  // parity of the CTA's groups (scans)
@@ -377,7 +374,7 @@ __device__ __forceinline__ void star_fx_consume(unsigned char *sm, const unsigne
     }
     const unsigned ob_idx = outb[st * NB + bs];
     const bool active = ok && ob_idx != 0xFFFFFFFFu;
-    double *buf = reinterpret_cast<double *>(sm + (st * NB + bs) * C::BRICK);
+    const double *buf = reinterpret_cast<const double *>(sm + (st * NB + bs) * C::BRICK);
     auto release = [&] {
       __syncwarp();
       if (lane == 0) mbar_arrive(empty0 + 8 * st);
@@ -385,42 +382,24 @@ __device__ __forceinline__ void star_fx_consume(unsigned char *sm, const unsigne
     int E = 0;
     bool stopped = false;
     // (a thread that gives up says so at the brick's first barrier, and its 64 threads stop)
-    const bool fx = fx_prepare(share, buf, TILE ? tile : buf, tp.fx, scan + 2 * NB * par, bs, E, active, !ok, stopped,
-                               [&] {
-                                 if constexpr (TILE) release();
-                               });
+    const bool fx = fx_prepare(share, buf, tile, tp.fx, scan + 2 * NB * par, bs, E, active, !ok, stopped, release);
     if (stopped) break;
     if (active) {
       double *out = reinterpret_cast<double *>(a.out) + a.out_off + (size_t)ob_idx * a.out_step;
       if (fx) {
         double *o = out + pk * 64 + pj * 8 + pi;
         const bool two = (reinterpret_cast<uintptr_t>(o) & 15) == 0;  // output bricks may start anywhere
-        auto put = [&](int k, double y0, double y1) {
-          if (two) st_pair(o + k * 64, make_double2(y0, y1));
-          else {
-            store_stream(o + k * 64, y0);
-            store_stream(o + k * 64 + 1, y1);
-          }
-        };
-        const int scale = fx_scale<60>(E, tp.fx.q);
-        if constexpr (TILE) {
-          typedef FxTile<R> X;
-          const double *c = tile + X::at(pk, pj, pi);
-          fx_star_pairs<R, SUM>([&](int k, int dj, int m) { return ld_pair(c + k * X::SK + dj * X::SJ + 2 * m); },
-                                [&](int k, int di) { return c[k * X::SK + di]; }, put, tp.fx, scale);
-        } else {
-          auto at = [&](int k, int j, int i) {  // one of the coordinates may lie in a face
-            return k < 0    ? 512 + ((k + R) * 8 + j) * 8 + i
-                   : k >= 8 ? 512 + 64 * R + ((k - 8) * 8 + j) * 8 + i
-                   : j < 0  ? 512 + 128 * R + (k * R + j + R) * 8 + i
-                   : j >= 8 ? 512 + 192 * R + (k * R + j - 8) * 8 + i
-                   : i < 0  ? 512 + 256 * R + (k * 8 + j) * IW + IW + i
-                   : i >= 8 ? 512 + 256 * R + 64 * IW + (k * 8 + j) * IW + i - 8
-                            : (k * 8 + j) * 8 + i;
-          };
-          fx_star_pairs<R, SUM>([&](int k, int dj, int m) { return ld_pair(buf + at(pk + k, pj + dj, pi + 2 * m)); },
-                                [&](int k, int di) { return buf[at(pk + k, pj, pi + di)]; }, put, tp.fx, scale);
-        }
+        fx_star_pairs<R, SUM>(
+            [&](int k, int dj, int m) { return ld_pair((k < 0 ? c0 : k < 4 ? c1 : c2) + k * X::SK + dj * X::SJ + 2 * m); },
+            [&](int k, int di) { return c1[k * X::SK + di]; },
+            [&](int k, double y0, double y1) {
+              if (two) st_pair(o + k * 64, make_double2(y0, y1));
+              else {
+                store_stream(o + k * 64, y0);
+                store_stream(o + k * 64 + 1, y1);
+              }
+            },
+            tp.fx, fx_scale<60>(E, tp.fx.q));
       } else {
         // FP64: one column per thread; its offsets are found here (kept out of the loop's registers)
         int l = lt;
@@ -428,12 +407,7 @@ __device__ __forceinline__ void star_fx_consume(unsigned char *sm, const unsigne
         star_column_f64_of<C, R>(buf, l, out, reinterpret_cast<const double *>(sm + S * NB * C::BRICK + C::O_COEF));
       }
     }
-    if (!(TILE && fx)) {
-      // an in-place conversion wrote the stage through the generic proxy; order those writes before
-      // the copies that refill it
-      if constexpr (!TILE) fence_proxy_async_smem();
-      release();
-    }
+    if (!fx) release();
     if (++st == S) {
       st = 0;
       ph ^= 1u;
@@ -676,7 +650,8 @@ int launch_star_tma(const SweepArgs &a, const Taps &tp, int dtype, cudaStream_t 
   typedef StarTmaCfg<T, BK, BJ, BI, R, NI> C;
   // default depth 2: on GB300 more resident CTAs beat deeper pipelines (FP32 star7 at 512^3:
   // 602 / 490 GStencil/s with 2 / 3 stages)
-  const int S = tma_stages(2);
+  // (fixed point of radius 4: one, which goes back as soon as it is read; with two a CTA less fits)
+  const int S = tma_stages(R == 4 && C::fx_tile(ACC) ? 1 : 2);
   const int smem = C::smem(S, ACC);
   if (smem > 227 * 1024) return fail(BK_ERR_UNSUPPORTED, "TMA sweep stage buffers exceed shared memory");
   TmaMaps maps;
