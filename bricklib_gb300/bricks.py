@@ -17,6 +17,7 @@ Dimension lists passed to init_grid / copyToBrick / copyFromBrick are contiguous
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from dataclasses import dataclass
 from typing import Optional, Sequence, Tuple
 
@@ -26,6 +27,7 @@ from . import _abi
 from ._abi import BK_BF16, BK_F32, BK_F64, call, lib
 from .stencils import Stencil
 
+_PACK3 = struct.Struct("3i").pack
 NP_DTYPE = {BK_F64: np.float64, BK_F32: np.float32, BK_BF16: np.uint16}
 ELEM_SIZE = {BK_F64: 8, BK_F32: 4, BK_BF16: 2}
 DTYPE_NAMES = {"f64": BK_F64, "f32": BK_F32, "bf16": BK_BF16}
@@ -184,7 +186,8 @@ class Layout:
         return int(np.prod(self.bdim))
 
     def to_c(self) -> _abi.bk_layout:
-        return _abi.bk_layout((C.c_int * 3)(*self.bdim), (C.c_int * 3)(*self.fold))
+        # packed rather than assigned member by member: each sweep makes one (2.7 against 0.9 us)
+        return _abi.bk_layout.from_buffer_copy(_PACK3(*self.bdim) + _PACK3(*self.fold))
 
     def offsets(self) -> np.ndarray:
         """layout(k, j, i) for every element in row-major (k, j, i) order
@@ -342,7 +345,7 @@ class Brick:
 
     def field(self) -> _abi.bk_field:
         s = self.bStorage
-        return _abi.bk_field(C.c_void_p(s.ptr), s.chunks, s.step, self.offset, s.dtype)
+        return _abi.bk_field(s.ptr, s.chunks, s.step, self.offset, s.dtype)
 
     def host_bricks(self) -> np.ndarray:
         """[chunks, BRICKSIZE] view of this field in host storage, layout order."""
@@ -452,8 +455,8 @@ def brickSweep(bIn: Brick, bOut: Brick, blist: BrickList, st, acc: int = _abi.BK
     """One sweep of stencil `st` over the bricks in `blist` (bk_sweep)."""
     cst = st if isinstance(st, _abi.bk_stencil) else to_c_stencil(st)
     info = bIn.bInfo
-    call("bk_sweep", C.c_void_p(info.ptr), info.nbricks, C.byref(bIn.field()), C.byref(bOut.field()),
-         C.c_void_p(blist.ptr), blist.n, C.byref(cst), C.byref(bIn.layout.to_c()), acc, stream_ptr(stream))
+    call("bk_sweep", info.ptr, info.nbricks, C.byref(bIn.field()), C.byref(bOut.field()), blist.ptr, blist.n,
+         C.byref(cst), C.byref(bIn.layout.to_c()), acc, stream_ptr(stream))
 
 
 def sweepKernel(bIn: Brick, bOut: Brick, st, acc: int = _abi.BK_ACC_NATIVE) -> str:
@@ -493,8 +496,7 @@ class GhostPlan:
 
 
 def ghostFill(plan: GhostPlan, brick: Brick, stream=None) -> None:
-    call("bk_ghost_fill", C.c_void_p(plan.ptr), plan.n, C.byref(brick.field()), C.byref(brick.layout.to_c()),
-         stream_ptr(stream))
+    call("bk_ghost_fill", plan.ptr, plan.n, C.byref(brick.field()), C.byref(brick.layout.to_c()), stream_ptr(stream))
 
 
 def timeSteps(a: Brick, b: Brick, blist: BrickList, st, steps: int, plan: Optional[GhostPlan] = None,
@@ -503,10 +505,9 @@ def timeSteps(a: Brick, b: Brick, blist: BrickList, st, steps: int, plan: Option
     current input every `fill_every` steps; returns the Brick holding the newest values."""
     cst = st if isinstance(st, _abi.bk_stencil) else to_c_stencil(st)
     info = a.bInfo
-    call("bk_steps", C.c_void_p(info.ptr), info.nbricks, C.byref(a.field()), C.byref(b.field()),
-         C.c_void_p(blist.ptr), blist.n, C.c_void_p(plan.ptr if plan else 0), plan.n if plan else 0,
-         C.byref(cst), C.byref(a.layout.to_c()), acc, steps, fill_every if plan else 0, 1 if use_graph else 0,
-         stream_ptr(stream))
+    call("bk_steps", info.ptr, info.nbricks, C.byref(a.field()), C.byref(b.field()), blist.ptr, blist.n,
+         plan.ptr if plan else None, plan.n if plan else 0, C.byref(cst), C.byref(a.layout.to_c()), acc, steps,
+         fill_every if plan else 0, 1 if use_graph else 0, stream_ptr(stream))
     return a if steps % 2 == 0 else b
 
 

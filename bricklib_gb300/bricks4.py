@@ -107,7 +107,7 @@ def sweep4(adj_dev: B.DeviceBuffer, nbricks: int, storage: B.BrickStorage, in_of
     """One 4-D sweep of `st` over the bricks in `blist` (bk_sweep4)."""
     cst = st if isinstance(st, bk_stencil4) else to_c_stencil4(st)
     so = out_storage or storage
-    fin = _abi.bk_field(C.c_void_p(storage.ptr), storage.chunks, storage.step, in_off, storage.dtype)
-    fout = _abi.bk_field(C.c_void_p(so.ptr), so.chunks, so.step, out_off, so.dtype)
-    call("bk_sweep4", C.c_void_p(adj_dev.ptr), nbricks, C.byref(fin), C.byref(fout), C.c_void_p(blist.ptr),
-         blist.n, C.byref(cst), C.byref(lay.to_c()), B.stream_ptr(stream))
+    fin = _abi.bk_field(storage.ptr, storage.chunks, storage.step, in_off, storage.dtype)
+    fout = _abi.bk_field(so.ptr, so.chunks, so.step, out_off, so.dtype)
+    call("bk_sweep4", adj_dev.ptr, nbricks, C.byref(fin), C.byref(fout), blist.ptr, blist.n, C.byref(cst),
+         C.byref(lay.to_c()), B.stream_ptr(stream))
