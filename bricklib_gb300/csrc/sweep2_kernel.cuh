@@ -27,6 +27,11 @@ __device__ __forceinline__ unsigned smem_u32(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
 }
 
+template <int N>
+struct Int {
+  static constexpr int value = N;
+};
+
 template <int BYTES>
 __device__ __forceinline__ void cp_async(unsigned dst, const void *src) {
   if (BYTES == 16)
@@ -147,6 +152,14 @@ __host__ __device__ constexpr int conflict_free_row(int need, int bi, int es, in
 #endif
 constexpr int PAIR_NB = BK_PAIR_NB;
 
+// A brick staged for its gather: the addresses of its 27 neighbour bricks (adjacency order, 13 the
+// brick itself) in the input field and of its brick in the output field, and whether it runs.
+struct __align__(16) Staged {
+  const unsigned char *src[27];
+  unsigned char *out;
+  unsigned long long active, pad;
+};
+
 // IST: the class-sum stream of the mirror-symmetric cubes (sym_cube_istream for FP64,
 // sym_cube_istream4 for 4- and 2-byte storage), one warp per 8x8x8 brick (two for the
 // compensated 4- and 2-byte stream, one row per thread).
@@ -211,10 +224,15 @@ struct Sweep2Cfg {
   static constexpr int NV_CUBE = HALO4 ? NV_ROWS + 2 * EK * EJ : EK * EJ * (NEED / VE);  // the row padding is never fetched
   static constexpr int NV = FAM == FAM_STAR ? NV_STAR : NV_CUBE;
   static constexpr int EPT = (NV + TPB - 1) / TPB;  // plan entries per thread
+  // copies whose source addresses are read together.  GB300 at 512^3, us, one / two / three / four:
+  // FP32 cube125 460 / 454 / 455 / 460, FP64 cube125 2199 / 2161 / 2159 / 2154, BF16 cube125 376 / 378 /
+  // 381 / 384; the other 4- and 2-byte kernels, whose warps are many, one: FP32 cube27 425 / 447, BF16
+  // 304 / 312
+  static constexpr int ISSUE = IST || ES == 8 ? 2 : 1;
   // float-float converts each raw FP64 tile into float pairs in place (same 8 bytes)
   static constexpr int FTILE_BYTES = 0;
   // bricks per CTA: as many as fit 128 threads and a ~100 KB shared-memory budget
-  static constexpr int PER_BRICK = 2 * TILE_BYTES + FTILE_BYTES + 3 * 36 * 4;
+  static constexpr int PER_BRICK = 2 * TILE_BYTES + FTILE_BYTES + 3 * (int)sizeof(Staged);
   static constexpr int NB = CS4 || FX125 ? 1 : PAIR ? PAIR_NB : cmax(1, cmin(cmax(1, 128 / TPB), (100 * 1024) / PER_BRICK));
   static constexpr int NT = TPB * NB;
   // native FP64 arithmetic on register operands (F64Ops).  Stars and cubes read them from a
@@ -232,10 +250,11 @@ struct Sweep2Cfg {
   static constexpr int SMEM = NB * PER_BRICK + COEFB + SCANB;
   // resident CTAs asked of the register allocator: the native FP32 / BF16 class-sum stream
   // (one warp per CTA) at <= 170 registers fits three warps per scheduler (12 per SM), which its
-  // shared memory also allows; the compensated stream (two warps per CTA): BK_CS_COMP_MINB
+  // shared memory also allows (radius 1, whose tile and sums are smaller: 16 -- FP32 at 512^3,
+  // 307 us against 331); the compensated stream (two warps per CTA): BK_CS_COMP_MINB
   // the fixed-point cubes: radius 1 five CTAs of two bricks (256^3: 236 us; four 244, three 261),
   // the 125-point one six of one brick (298 us; seven 301 with fewer registers)
-  static constexpr int MINB = CS4 ? (ACC == ACCM_NATIVE ? 12 : BK_CS_COMP_MINB) : FX125 ? 6 : FX && FAM == FAM_CUBE ? 5 : 0;
+  static constexpr int MINB = CS4 ? (ACC == ACCM_NATIVE ? (R == 1 ? 16 : 12) : BK_CS_COMP_MINB) : FX125 ? 6 : FX && FAM == FAM_CUBE ? 5 : 0;
 };
 
 // Tile coordinates (kk, jj, ii) of plan vector g for the star / cube neighbourhood.
@@ -1310,19 +1329,16 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char *raw0 = smem_raw;                               // [NB] tiles, buffer 0
   unsigned char *raw1 = smem_raw + NB * C::TILE_BYTES;          // [NB] tiles, buffer 1
-  unsigned *nbrs = reinterpret_cast<unsigned *>(smem_raw + 2 * NB * C::TILE_BYTES + NB * C::FTILE_BYTES);
-  // nbrs slot (36 words): [0..26] adjacency, [27] active, [28..29] input field base,
-  // [30..31] output field base, [32..33] / [34..35] input / output storage step (elements)
-  // nbrs: [3][NB][28]: adjacency of the groups being computed, copied and staged
-  // (three slots, so staging the group after next never overwrites one still read);
-  // entry [27] is the brick's active flag
+  // [3][NB]: the bricks of the groups being computed, copied and staged (three slots, so staging
+  // the group after next never overwrites one still read)
+  Staged *nbrs = reinterpret_cast<Staged *>(smem_raw + 2 * NB * C::TILE_BYTES + NB * C::FTILE_BYTES);
 
   const int slot = threadIdx.x / TPB, lt = threadIdx.x - slot * TPB;
   unsigned plan[EPT];
 #pragma unroll
   for (int e = 0; e < EPT; ++e) {
     const int g = e * TPB + lt;
-    plan[e] = g < C::NV ? plan_entry<C, BK, BJ, BI, R, FAM, IST>(g) : 0xFFFFFFFFu;
+    plan[e] = g < C::NV ? plan_entry<C, BK, BJ, BI, R, FAM, IST>(g) : 0u;
   }
 
   const long long ngroups = ((long long)a.nlist + NB - 1) / NB;
@@ -1356,122 +1372,134 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
                        : STREAM ? (long long)blockIdx.x * ngroups / G : (long long)blockIdx.x;
   const long long gend = STREAM && !CHUNKED ? ((long long)blockIdx.x + 1) * ngroups / G : ngroups;
 
-  // Adjacency of a group: fetched into registers two groups ahead (its global-load latency
-  // hides under the current group's compute), stored into one of three nbrs slots.
+  // List entry and adjacency of a group, in registers until they are stored to one of three nbrs
+  // slots: the entry is loaded three groups ahead, the adjacency two (its address is then at
+  // hand), and the range checks wait for the store, so that neither load is waited for.  With the
+  // entry, the adjacency and the checks in one place, a brick's warps stood still for two trips to
+  // memory: GB300, 512^3, FP32 cube125 519 -> 494 us, FP64 2272 -> 2238, BF16 cube27 326 -> 314.
   constexpr int APT = (27 + TPB - 1) / TPB;  // adjacency entries per thread
+  uint2 ent = make_uint2(0, 0);              // batch: domain, brick; plain: -, brick
   unsigned av[APT];
-  int aok[APT];
-  unsigned long long fin = 0, fout = 0, fsin = 0, fsout = 0;  // held by the thread of slot 13
+  bool alive = false, listed = false;  // the group has an entry here; its brick is in range
+  long long achunks = 0;               // batch: bricks of the domain's fields
+  // batch: the domain's fields and their bytes per brick
+  const unsigned char *fin = nullptr;
+  unsigned char *fout = nullptr;
+  unsigned long long fstep = 0;
+  auto fetch_entry = [&](long long grp) {
+    const long long n = grp * NB + slot;
+    if (grp < gend && n < a.nlist) {
+      if constexpr (BATCH) ent = a.work[n];
+      else ent.y = a.blist[n];
+    }
+  };
   auto fetch_adj = [&](long long grp) {
     const long long n = grp * NB + slot;
+    alive = grp < gend && n < a.nlist;
+    listed = false;
+    if (!alive) return;
+    const unsigned *adj = a.adj;
+    if constexpr (BATCH) {
+      const bool dok = ent.x < a.ndom;
+      const BatchDomain &D = a.doms[dok ? ent.x : 0];
+      adj = D.adj;
+      achunks = D.chunks;
+      listed = dok && ent.y < D.nbricks;
+      fin = reinterpret_cast<const unsigned char *>(a.parity ? D.f1 : D.f0);
+      fout = reinterpret_cast<unsigned char *>(a.parity ? D.f0 : D.f1);
+      fstep = D.step_bytes;
+    } else {
+      listed = ent.y < a.nbricks;
+    }
+    if (listed) {
 #pragma unroll
-    for (int q = 0; q < APT; ++q) {
-      const int sl = lt + q * TPB;
-      unsigned v = 0;
-      int ok = 0;
-      if (sl < 27 && grp < gend && n < a.nlist) {
-        const unsigned *adj;
-        unsigned b, nbricks;
-        long long in_chunks, out_chunks;
-        if constexpr (BATCH) {
-          const uint2 w = a.work[n];
-          const bool dok = w.x < a.ndom;
-          const BatchDomain &D = a.doms[dok ? w.x : 0];
-          adj = D.adj;
-          b = dok ? w.y : 0xFFFFFFFFu;
-          nbricks = D.nbricks;
-          in_chunks = out_chunks = D.chunks;
-          if (sl == 13) {
-            fin = reinterpret_cast<unsigned long long>(a.parity ? D.f1 : D.f0);
-            fout = reinterpret_cast<unsigned long long>(a.parity ? D.f0 : D.f1);
-            fsin = fsout = D.step_bytes / sizeof(T);
-          }
-        } else {
-          adj = a.adj;
-          b = a.blist[n];
-          nbricks = a.nbricks;
-          in_chunks = a.in_chunks;
-          out_chunks = a.out_chunks;
-          if (sl == 13) {
-            fin = reinterpret_cast<unsigned long long>(reinterpret_cast<const T *>(a.in) + a.in_off);
-            fout = reinterpret_cast<unsigned long long>(reinterpret_cast<T *>(a.out) + a.out_off);
-            fsin = a.in_step;
-            fsout = a.out_step;
-          }
-        }
-        if (b < nbricks) {
-          v = adj[(size_t)b * 27 + sl];
-          ok = 1;
-          if (sl == 13 && ((long long)v >= out_chunks || (long long)v >= in_chunks)) ok = 0;
-          if ((long long)v >= in_chunks || !ok) { atomicOr(a.err, FLAG_BOUNDS); v = 0; }
-        } else if (sl == 13) {
-          atomicOr(a.err, FLAG_BOUNDS);
-        }
+      for (int q = 0; q < APT; ++q) {
+        const int sl = lt + q * TPB;
+        if (sl < 27) av[q] = adj[(size_t)ent.y * 27 + sl];
       }
-      av[q] = v;
-      aok[q] = ok;
     }
   };
   auto store_adj = [&](int ns) {
-    unsigned *nbr = nbrs + (ns * NB + slot) * 36;
+    Staged &nb = nbrs[ns * NB + slot];
+    const long long in_chunks = BATCH ? achunks : a.in_chunks, out_chunks = BATCH ? achunks : a.out_chunks;
+    const unsigned char *in =
+        BATCH ? fin : reinterpret_cast<const unsigned char *>(reinterpret_cast<const T *>(a.in) + a.in_off);
+    const size_t in_step = BATCH ? fstep : a.in_step * sizeof(T);
 #pragma unroll
     for (int q = 0; q < APT; ++q) {
       const int sl = lt + q * TPB;
       if (sl < 27) {
-        nbr[sl] = av[q];
+        unsigned v = listed ? av[q] : 0u;
+        bool ok = listed;
+        if (listed) {
+          if (sl == 13 && (long long)v >= out_chunks) ok = false;
+          if ((long long)v >= in_chunks) ok = false;
+          if (!ok) {  // a neighbour out of range reads brick 0, a centre out of range does not run
+            atomicOr(a.err, FLAG_BOUNDS);
+            v = 0;
+          }
+        } else if (alive && sl == 13) {
+          atomicOr(a.err, FLAG_BOUNDS);
+        }
+        nb.src[sl] = in + v * in_step;
         if (sl == 13) {
-          nbr[27] = aok[q];
-          *reinterpret_cast<unsigned long long *>(nbr + 28) = fin;
-          *reinterpret_cast<unsigned long long *>(nbr + 30) = fout;
-          *reinterpret_cast<unsigned long long *>(nbr + 32) = fsin;
-          *reinterpret_cast<unsigned long long *>(nbr + 34) = fsout;
+          nb.active = ok;
+          nb.out = BATCH ? fout + v * fstep
+                         : reinterpret_cast<unsigned char *>(reinterpret_cast<T *>(a.out) + a.out_off + v * a.out_step);
         }
       }
     }
   };
-  // issue the asynchronous gather of the group staged in nbrs[ns] into raw buffer buf
-  // Whether the stream continues from the group whose adjacency is in nbrs[prev] into the group
-  // in nbrs[ns]: both ran, and the latter's i-lo and centre columns of neighbours are the
-  // former's centre and i-hi columns (lanes 0..17 of every warp check one slot pair each, so
-  // all warps of a brick reach the same answer).
+  // Whether the stream continues from the group staged in nbrs[prev] into the group in nbrs[ns]:
+  // both ran, and the latter's i-lo and centre columns of neighbours are the former's centre and
+  // i-hi columns (lanes 0..17 of every warp check one slot pair each, so all warps of a brick
+  // reach the same answer).  The addresses are compared, so in batch mode a stream never runs from
+  // one domain's field into another's.
   auto continues = [&](int prev, int ns) -> bool {
-    const unsigned *nb = nbrs + ns * 36, *pv = nbrs + prev * 36;
+    const Staged &nb = nbrs[ns], &pv = nbrs[prev];
     bool same = true;
     const int wl = lt & 31;
     if (wl < 18) {
       const int s9 = wl < 9 ? wl : wl - 9, sh = wl < 9 ? 0 : 1;
       const int base = (s9 / 3) * 9 + (s9 % 3) * 3;  // (dk, dj) = (s9 / 3 - 1, s9 % 3 - 1), di = -1
-      same = nb[base + sh] == pv[base + sh + 1];
+      same = nb.src[base + sh] == pv.src[base + sh + 1];
     }
-    // the same input field: in batch mode consecutive items may belong to different domains
-    same = same && *reinterpret_cast<const unsigned long long *>(nb + 28) ==
-                       *reinterpret_cast<const unsigned long long *>(pv + 28);
-    return __all_sync(0xFFFFFFFFu, same) && pv[27] != 0 && nb[27] != 0;
+    return __all_sync(0xFFFFFFFFu, same) && pv.active && nb.active;
   };
   // issue the asynchronous gather of the group staged in nbrs[ns] into raw buffer buf; a
   // continued stream reads only the tile columns from ICUT on (the W of the columns before
   // come from the previous brick), so copies wholly before ICUT are skipped
   // plan entries a continued brick issues: those of the first NVN copies (warp-uniform bound)
   constexpr int EPTN = STREAM ? (StreamPlan<C, R>::NVN + TPB - 1) / TPB : EPT;
-  auto issue = [&](int buf, int ns, bool cont) {
-    const unsigned *nbr = nbrs + (ns * NB + slot) * 36;
-    if (nbr[27]) {
-      unsigned char *tile = (buf ? raw1 : raw0) + slot * C::TILE_BYTES;
-      const unsigned tbase = smem_u32(tile);
-      const T *in = reinterpret_cast<const T *>(*reinterpret_cast<const unsigned long long *>(nbr + 28));
-      const size_t step = *reinterpret_cast<const unsigned long long *>(nbr + 32);
-      const int ne = STREAM && cont ? EPTN : EPT;
+  // copies [E0, E1) of this thread: the neighbours' addresses are read from shared memory ISSUE
+  // copies at a time, ahead of the copies, which the compiler keeps in order with every access (a
+  // brick index read and multiplied out in front of each copy: GB300, 512^3, FP32 cube125 494 us
+  // against 454, FP64 2238 against 2161, BF16 424 against 378)
+  auto copies = [&](auto first, auto last, const Staged &nb, unsigned tbase) {
+    constexpr int E0 = decltype(first)::value, E1 = decltype(last)::value, STEP = C::ISSUE;
 #pragma unroll
-      for (int e = 0; e < EPT; ++e) {
-        const unsigned p = plan[e];
-        const bool need = !(STREAM && cont) || e * TPB + lt < StreamPlan<C, R>::NVN;
-        if (e < ne && need && p != 0xFFFFFFFFu) {
-          const unsigned sl = p & 31u, src = (p >> 5) & 8191u, dst = p >> 18;
-          const T *g = in + (size_t)nbr[sl] * step + src;
-          if (C::HALO4 && e * TPB + lt >= C::NV_ROWS) cp_async<4>(tbase + dst * C::ES, g);
-          else cp_async<C::VB>(tbase + dst * C::ES, g);
+    for (int e0 = E0; e0 < E1; e0 += STEP) {
+      const unsigned char *g[STEP];
+#pragma unroll
+      for (int x = 0; x < STEP; ++x)
+        if (e0 + x < E1) g[x] = nb.src[plan[e0 + x] & 31u] + ((plan[e0 + x] >> 5) & 8191u) * (unsigned)C::ES;
+#pragma unroll
+      for (int x = 0; x < STEP; ++x) {
+        const int e = e0 + x;
+        if (e < E1 && e * TPB + lt < (E1 == EPT ? C::NV : StreamPlan<C, R>::NVN)) {
+          const unsigned dst = tbase + (plan[e] >> 18) * (unsigned)C::ES;
+          if (C::HALO4 && e * TPB + lt >= C::NV_ROWS) cp_async<4>(dst, g[x]);
+          else cp_async<C::VB>(dst, g[x]);
         }
       }
+    }
+  };
+  auto issue = [&](int buf, int ns, bool cont) {
+    const Staged &nb = nbrs[ns * NB + slot];
+    if (nb.active) {
+      const unsigned tbase = smem_u32((buf ? raw1 : raw0) + slot * C::TILE_BYTES);
+      if (STREAM && cont) copies(Int<0>{}, Int<EPTN>{}, nb, tbase);
+      else copies(Int<0>{}, Int<EPT>{}, nb, tbase);
     }
     cp_async_commit();
   };
@@ -1496,9 +1524,12 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
   Walk w1{g0, 0};
   Walk w2 = advance(w1), w3 = advance(w2);  // the next group and the one after
   long long grp = g0;
+  fetch_entry(grp);
   fetch_adj(grp);
+  fetch_entry(w2.g);
   store_adj(0);
   fetch_adj(w2.g);
+  fetch_entry(w3.g);
   store_adj(1);
   __syncthreads();
   issue(0, 0, false);
@@ -1513,12 +1544,13 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
     const int ncur = it % 3, nnxt = (it + 1) % 3, nfar = (it + 2) % 3;
     __syncthreads();     // nbrs[nnxt] visible; every thread is done with raw[nxt] and nbrs[nfar]
     issue(nxt, nnxt, STREAM && continues(ncur, nnxt));
-    fetch_adj(w3.g);  // lands while this group computes
+    fetch_adj(w3.g);             // lands while this group computes
+    fetch_entry(advance(w3).g);  // lands by the next group's turn
     cp_async_wait<1>();  // this thread's copies for the current group have landed
     __syncthreads();     // ... and everybody else's
 
-    const unsigned *nbr = nbrs + (ncur * NB + slot) * 36;
-    const bool active = nbr[27] != 0;
+    const Staged &nbr = nbrs[ncur * NB + slot];
+    const bool active = nbr.active != 0;
     const T *rt = reinterpret_cast<const T *>((cur ? raw1 : raw0) + slot * C::TILE_BYTES);
     if constexpr (ACC == ACCM_FF) {
       // one pass, in place: raw doubles -> float pairs (each thread its own elements)
@@ -1535,9 +1567,7 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
       // ones a continued stream does not read)
       const bool cont = STREAM && it > 0 && continues(nfar, ncur);
       if (active) {
-        T *out = reinterpret_cast<T *>(*reinterpret_cast<const unsigned long long *>(nbr + 30));
-        const size_t ostep = *reinterpret_cast<const unsigned long long *>(nbr + 34);
-        T *ob = out + (size_t)nbr[13] * ostep;
+        T *ob = reinterpret_cast<T *>(nbr.out);
         T *tile = const_cast<T *>(rt);  // this brick's buffer until the next barrier
         if constexpr (C::ES == 8) {
           if (tp.kj) sym_cube_istream<C, R, true>(tile, ob, lt, tp, W, cont);
@@ -1549,13 +1579,11 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
         }
       }
     } else if (active) {
-      T *out = reinterpret_cast<T *>(*reinterpret_cast<const unsigned long long *>(nbr + 30));
-      const size_t ostep = *reinterpret_cast<const unsigned long long *>(nbr + 34);
+      T *ob = reinterpret_cast<T *>(nbr.out);
       if constexpr (C::FX) {
         int E = 0;
         bool stopped = false;
         double *tile = reinterpret_cast<double *>(const_cast<T *>(rt));
-        T *ob = out + (size_t)nbr[13] * ostep;
         if (fx_prepare(share, tile, tile, tp.fx, scan + 2 * NB * cur, slot, E, true, false, stopped, [] {}))
           sweep2_brick_fx<T, R, FAM, ACC>(tile, ob, lt, tp, E);
         else if constexpr (C::FX125)
@@ -1563,7 +1591,7 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
         else
           sweep2_brick<T, BK, BJ, BI, R, FAM, ACCM_NATIVE>(rt, ob, lt, tp, cs);
       } else
-        sweep2_brick<T, BK, BJ, BI, R, FAM, ACC>(rt, out + (size_t)nbr[13] * ostep, lt, tp, cs);
+        sweep2_brick<T, BK, BJ, BI, R, FAM, ACC>(rt, ob, lt, tp, cs);
     }
     store_adj(nfar);  // group it + 2; read after the next iteration's first barrier
   }
