@@ -304,13 +304,14 @@ static int plan_sweep(const bk_field *in, const bk_field *out, const bk_stencil 
     if (plan->fam == FAM_CUBE && plan->shape == 0 && !plan->out_pair) plan->v2 = false;
     // star stencils on 8x8x8 row-major bricks: the TMA-fed kernel, unless a kernel is forced
     plan->tma = tma_eligible(*plan, in) && !getenv("BK_SWEEP_ONESHOT") && !getenv("BK_SWEEP_PIPELINED");
-    // mirror-symmetric cubes: the pipelined kernel streams class sums along i -- FP64 in native
-    // arithmetic, FP32 / BF16 in native or compensated FP32 (BK_SWEEP_ISTREAM=0: one brick at a
+    // cubes: the pipelined kernel streams column sums along i -- mirror-symmetric ones as class sums,
+    // FP64 in native arithmetic, FP32 / BF16 in native or compensated FP32, and on FP32 / BF16 in
+    // native arithmetic the radius-1 cube without the symmetry (BK_SWEEP_ISTREAM=0: one brick at a
     // time on column pairs)
     const char *ist = getenv("BK_SWEEP_ISTREAM");
-    plan->istream = plan->v2 && plan->sym && plan->shape == 0 && !(ist && !strcmp(ist, "0")) &&
-                    (in->dtype == BK_F64 ? plan->acc == ACCM_NATIVE
-                                         : (plan->acc == ACCM_NATIVE || plan->acc == ACCM_COMP));
+    plan->istream = plan->v2 && plan->shape == 0 && !(ist && !strcmp(ist, "0")) &&
+                    (plan->sym ? plan->acc == ACCM_NATIVE || (in->dtype != BK_F64 && plan->acc == ACCM_COMP)
+                               : plan->fam == FAM_CUBE && plan->r == 1 && in->dtype != BK_F64 && plan->acc == ACCM_NATIVE);
   }
   *Lout = L;
   return BK_OK;

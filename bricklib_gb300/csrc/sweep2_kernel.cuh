@@ -131,8 +131,6 @@ __host__ __device__ constexpr int conflict_free_row(int need, int bi, int es, in
 #define BK_CS_SWZ 1
 #endif
 
-// bricks (warps) per CTA of the column-pair cube kernels: one, so that a CTA's barriers wait
-// for no other warp (GB300, FP32 cube125 at 512^3: 191 / 171 GStencil/s with one / two)
 // class-sum streams of 4- / 2-byte storage: about this many consecutive groups per chunk of a
 // CTA's walk
 #ifndef BK_CS_CHUNK
@@ -147,6 +145,8 @@ __host__ __device__ constexpr int conflict_free_row(int need, int bi, int es, in
 #define BK_CS_COMP_MINB 8
 #endif
 
+// bricks (warps) per CTA of the column-pair cube kernels: one, so that a CTA's barriers wait
+// for no other warp (GB300, FP32 cube125 at 512^3: 191 / 171 GStencil/s with one / two)
 #ifndef BK_PAIR_NB
 #define BK_PAIR_NB 1
 #endif
@@ -162,7 +162,8 @@ struct __align__(16) Staged {
 
 // IST: the class-sum stream of the mirror-symmetric cubes (sym_cube_istream for FP64,
 // sym_cube_istream4 for 4- and 2-byte storage), one warp per 8x8x8 brick (two for the
-// compensated 4- and 2-byte stream, one row per thread).
+// compensated 4- and 2-byte stream, one row per thread); and, on 4- and 2-byte storage, the stream of
+// the radius-1 cube without that symmetry (cube_istream4).
 template <typename T, int BK, int BJ, int BI, int R, int FAM, int ACC, bool IST = false>
 struct Sweep2Cfg {
   static constexpr int ES = (int)sizeof(T);
@@ -184,18 +185,14 @@ struct Sweep2Cfg {
   // (two-way within a half warp, which reads half the bytes of the FP32 case)
   static constexpr bool CS4 = IST && ES <= 4;
   static constexpr bool SWZ = BK_CS_SWZ && CS4 && ES == 4 && BI + 2 * RP == 16;
-  // the FP32 27-point cube on column pairs: rows of 12, the one halo value of either side by a 4-byte
-  // copy (low: before the centre; high: at the next row's front, unused there), half the tile of
-  // rows held as whole 16-byte copies and padded to 24: twice the resident CTAs
-  static constexpr bool HALO4 = ES == 4 && FAM == FAM_CUBE && R == 1 && BK == 8 && BJ == 8 && BI == 8 && ACC == ACCM_NATIVE;
-  static constexpr int EI = HALO4 ? BI + RP : CS4 ? (ES == 4 ? (SWZ ? 16 : 20) : 24)
+  static constexpr int EI = CS4 ? (ES == 4 ? (SWZ ? 16 : 20) : 24)
                           : PERM ? (NEED % 8 <= 4 ? NEED - NEED % 8 + 4 : NEED - NEED % 8 + 12)
                                  : conflict_free_row(NEED, BI, ES, VE);
   // the 125-point cube in fixed point: planes two elements longer, so that a quarter warp's pair loads
   // from four rows of two planes fall in different banks
   static constexpr bool FX125 = FAM == FAM_CUBE && R == 2 && ACC == ACCM_FXS;
   static constexpr int SK = EJ * EI + (FX125 ? 2 : 0);  // elements per plane
-  static constexpr int TILE = EK * SK + (HALO4 ? VE : 0);  // elements per brick tile
+  static constexpr int TILE = EK * SK;  // elements per brick tile
   // position within tile row jj of column ii (SWZ: the row's 16-byte units permuted)
   static __host__ __device__ __forceinline__ int col(int jj, int ii) {
     return SWZ ? ((((ii >> 2) ^ ((jj >> 1) & 3)) << 2) | (ii & 3)) : ii;
@@ -208,6 +205,9 @@ struct Sweep2Cfg {
   // cube125 191 / 156; BF16 cube27 412 / 302, cube125 235 / 139).
   static constexpr bool PAIR = BK == 8 && BJ == 8 && BI == 8 && ACC == ACCM_NATIVE &&
                                (FAM == FAM_CUBESYM || FAM == FAM_CUBESYM_IJ || (FAM == FAM_CUBE && R == 1 && ES <= 4));
+  // the radius-1 stream (cube_istream4) writes a brick with the next one's first columns: which halo
+  // columns a brick needs is known one brick further ahead
+  static constexpr bool DEFER = CS4 && FAM == FAM_CUBE;
   static constexpr bool WARP1 = PAIR || CS4;  // one warp per brick (the compensated stream: two)
   // rows of the brick per thread in the FP32 / BF16 class-sum stream: two in native arithmetic
   // (one warp per brick), one under compensated accumulation (two warps per brick), whose Dot2
@@ -220,10 +220,12 @@ struct Sweep2Cfg {
   static constexpr int NV_JF = BK * R * (BI / VE);   // one j face
   static constexpr int NV_IF = BK * BJ * (RP / VE);  // one i face
   static constexpr int NV_STAR = NV_CENTRE + 2 * (NV_KF + NV_JF + NV_IF);
-  static constexpr int NV_ROWS = EK * EJ * (BI / VE);  // HALO4: the centre rows, then two halo values a row
-  static constexpr int NV_CUBE = HALO4 ? NV_ROWS + 2 * EK * EJ : EK * EJ * (NEED / VE);  // the row padding is never fetched
+  static constexpr int NV_CUBE = EK * EJ * (NEED / VE);  // the row padding is never fetched
   static constexpr int NV = FAM == FAM_STAR ? NV_STAR : NV_CUBE;
-  static constexpr int EPT = (NV + TPB - 1) / TPB;  // plan entries per thread
+  // DEFER: the centre columns' copies, then the i-lo columns' (the i-hi ones follow from those)
+  static constexpr int NV_MID = EK * EJ * (BI / VE), NV_SIDE = EK * EJ * (RP / VE);
+  static constexpr int EPT_MID = (NV_MID + TPB - 1) / TPB, EPT_SIDE = (NV_SIDE + TPB - 1) / TPB;
+  static constexpr int EPT = DEFER ? EPT_MID + EPT_SIDE : (NV + TPB - 1) / TPB;  // plan entries per thread
   // copies whose source addresses are read together.  GB300 at 512^3, us, one / two / three / four:
   // FP32 cube125 460 / 454 / 455 / 460, FP64 cube125 2199 / 2161 / 2159 / 2154, BF16 cube125 376 / 378 /
   // 381 / 384; the other 4- and 2-byte kernels, whose warps are many, one: FP32 cube27 425 / 447, BF16
@@ -248,27 +250,20 @@ struct Sweep2Cfg {
   static constexpr int COEFB = F64S ? ((F64Ops::NHEAD + NCOEF) * 8 + 15) / 16 * 16 : 0;
   static constexpr int SCANB = FX ? 2 * NB * 2 * 8 : 0;  // fixed-point scans, [call parity][brick][warp] int2
   static constexpr int SMEM = NB * PER_BRICK + COEFB + SCANB;
-  // resident CTAs asked of the register allocator: the native FP32 / BF16 class-sum stream
-  // (one warp per CTA) at <= 170 registers fits three warps per scheduler (12 per SM), which its
-  // shared memory also allows (radius 1, whose tile and sums are smaller: 16 -- FP32 at 512^3,
-  // 307 us against 331); the compensated stream (two warps per CTA): BK_CS_COMP_MINB
+  // resident CTAs asked of the register allocator: the native FP32 / BF16 class-sum stream (one warp
+  // per CTA) 11, as many as the FP32 tiles leave room for (512^3, us, 10 / 11 / 12 / 13: FP32 453 / 454 /
+  // 483 / 490, BF16 377 / 377 / 377 / 429), with radius 1, whose tile and sums are smaller, 16 (FP32
+  // 307 against 331 for 12) and without the symmetry 14 (FP32 291, 295 for 16; BF16 16: 241, 244
+  // for 14); the compensated stream (two warps per CTA): BK_CS_COMP_MINB
   // the fixed-point cubes: radius 1 five CTAs of two bricks (256^3: 236 us; four 244, three 261),
   // the 125-point one six of one brick (298 us; seven 301 with fewer registers)
-  static constexpr int MINB = CS4 ? (ACC == ACCM_NATIVE ? (R == 1 ? 16 : 12) : BK_CS_COMP_MINB) : FX125 ? 6 : FX && FAM == FAM_CUBE ? 5 : 0;
+  static constexpr int MINB = CS4 ? (ACC == ACCM_NATIVE ? (R > 1 ? 11 : DEFER && ES == 4 ? 14 : 16) : BK_CS_COMP_MINB) : FX125 ? 6 : FX && FAM == FAM_CUBE ? 5 : 0;
 };
 
 // Tile coordinates (kk, jj, ii) of plan vector g for the star / cube neighbourhood.
 template <typename C, int BK, int BJ, int BI, int R, int FAM>
 __device__ __forceinline__ void plan_coords(int g, int &kk, int &jj, int &ii) {
   constexpr int VE = C::VE, RP = C::RP;
-  if constexpr (C::HALO4) {
-    const bool halo = g >= C::NV_ROWS;
-    const int h = g - C::NV_ROWS, row = halo ? h >> 1 : g / (BI / VE);
-    kk = row / C::EJ;
-    jj = row % C::EJ;
-    ii = halo ? ((h & 1) ? RP + BI : RP - 1) : RP + (g % (BI / VE)) * VE;
-    return;
-  }
   if (FAM != FAM_STAR) {
     constexpr int RV = C::NEED / VE;
     kk = g / (C::EJ * RV);
@@ -341,7 +336,14 @@ struct StreamPlan {
 template <typename C, int BK, int BJ, int BI, int R, int FAM, bool SORD = false>
 __device__ __forceinline__ unsigned plan_entry(int g) {
   int kk, jj, ii;
-  if constexpr (SORD) {
+  if constexpr (C::DEFER) {
+    const bool side = g >= C::EPT_MID * C::TPB;
+    const int rv = (side ? C::RP : BI) / C::VE, n = side ? C::NV_SIDE : C::NV_MID;
+    const int y = g - (side ? C::EPT_MID * C::TPB : 0), x = y < n ? y : 0;
+    kk = x / rv / C::EJ;
+    jj = x / rv % C::EJ;
+    ii = (side ? 0 : C::RP) + x % rv * C::VE;
+  } else if constexpr (SORD) {
     typedef StreamPlan<C, R> P;
     static_assert(FAM != FAM_STAR, "streams are for cubes");
     int row, chunk;
@@ -864,9 +866,29 @@ __device__ __forceinline__ void cs_shift(CsWin<R, COMP, NO> &S, const float2 (&W
       }
 }
 
+// A brick's outputs, parked from tile column c0 on, leave in whole-warp stores (16 / 8 bytes per lane) when the output brick
+// is aligned for them.
+template <typename C, int R, typename T>
+__device__ __forceinline__ void cs_store(const T *rt, T *ob, const int lane, const int c0 = C::RP) {
+  constexpr int SK = C::EJ * C::EI, SJ = C::EI, TPB = C::TPB;
+  constexpr int AL = 4 * (int)sizeof(T);
+  if ((reinterpret_cast<uintptr_t>(ob) & (AL - 1)) == 0) {
+#pragma unroll
+    for (int q = 0; q < 512 / (4 * TPB); ++q) {
+      const int e = q * 4 * TPB + 4 * lane, k = e >> 6, jj = (e >> 3) & 7, i = e & 7;
+      st_quad(ob + e, rt + (k + R) * SK + (jj + R) * SJ + C::col(jj + R, c0 + i));
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 512 / TPB; ++q) {
+      const int e = q * TPB + lane, k = e >> 6, jj = (e >> 3) & 7, i = e & 7;
+      ob[e] = rt[(k + R) * SK + (jj + R) * SJ + C::col(jj + R, c0 + i)];
+    }
+  }
+}
+
 // One brick of the stream: its eight output columns (groups at tile columns RP and RP + 4), the
-// W of groups RP - 4 and RP computed here unless the stream continues (cont), then the brick
-// leaves in whole-warp stores (16 / 8 bytes per lane) when the output brick is aligned for them.
+// W of groups RP - 4 and RP computed here unless the stream continues (cont).
 // A thread (lane of the brick's TPB threads) owns rows (k0 .. k0 + NO - 1, j); with two warps per
 // brick the syncs around the parking are block barriers.
 template <typename C, typename T, int R, bool KJ, bool COMP>
@@ -896,19 +918,143 @@ __device__ __forceinline__ void sym_cube_istream4(T *rt, T *ob, const int lane, 
   cs_out<C, T, R, COMP, NO>(park, j + R, RP + 4, S, Wn, En);
   cs_shift<R, COMP, NO>(S, Wn, En);
   sync();  // the parked outputs of every thread are in the tile
-  constexpr int AL = 4 * (int)sizeof(T);
-  if ((reinterpret_cast<uintptr_t>(ob) & (AL - 1)) == 0) {
+  cs_store<C, R>(rt, ob, lane);
+}
+
+// The radius-1 cube without mirror symmetry on 4- and 2-byte storage, streamed along i like the
+// class sums: the same tile, rows and loads, one weighted sum of the 3 x 3 values of a column per
+// tap offset d along i,
+//   W_d(i) = sum over dk, dj of coef(dk, dj, d) x(k + dk, j + dj, i)     d = -1, 0, 1
+//   out(i) = (W_-1(i - 1) + W_0(i)) + W_1(i + 1)
+// in packed FP32 (27 FFMA2 per column pair).  A brick's last outputs want the first column of the
+// brick after it: where the stream goes on they wait for that brick, which then writes both halves
+// of every row, and the i-hi columns are never fetched -- a run of bricks fetches every column once.
+// Bound by the gathers and their latency: a column pair per lane over its whole brick, with the halo
+// values either side of a row fetched for every brick, ran at 424 us (FP32, 512^3, 281 here) and 305
+// (BF16, 239); writing every brick at once, with its i-hi columns, at 300 and 284.  A shuffled list,
+// 320^3, here and on column pairs: FP32 122 us, 128, BF16 88, 87; grid order 82, 113 and 66, 86.
+template <int NO>
+struct RunWin {
+  float head[NO][4];           // the brick's first four outputs of a row
+  float part[NO][4], last[NO];  // the window's outputs, the last short of W_1; W_-1 of its last column
+};
+
+// W_d of the one column c (a brick's i-lo or i-hi one), d = D - 1
+template <typename C, typename T, int NO, int D>
+__device__ __forceinline__ void run_edge(const T *base, const int j, const int c, const Taps &tp, float (&w)[NO]) {
+  constexpr int SK = C::EJ * C::EI, SJ = C::EI;
 #pragma unroll
-    for (int q = 0; q < 512 / (4 * TPB); ++q) {
-      const int e = q * 4 * TPB + 4 * lane, k = e >> 6, jj = (e >> 3) & 7, i = e & 7;
-      st_quad(ob + e, rt + (k + R) * SK + (jj + R) * SJ + C::col(jj + R, RP + i));
-    }
-  } else {
+  for (int q = 0; q < 2 + NO; ++q)
 #pragma unroll
-    for (int q = 0; q < 512 / TPB; ++q) {
-      const int e = q * TPB + lane, k = e >> 6, jj = (e >> 3) & 7, i = e & 7;
-      ob[e] = rt[(k + R) * SK + (jj + R) * SJ + C::col(jj + R, RP + i)];
+    for (int rr = 0; rr < 3; ++rr) {
+      const float x = to_acc(base[q * SK + rr * SJ + C::col(j + rr, c)]);
+#pragma unroll
+      for (int o = 0; o < NO; ++o) {
+        const int dk = q - o;
+        if (dk < 0 || dk > 2) continue;
+        const float cf = tp.cf[(dk * 3 + rr) * 3 + D];
+        w[o] = dk == 0 && rr == 0 ? cf * x : fmaf(cf, x, w[o]);
+      }
     }
+}
+
+template <typename C, typename T, int NO>
+__device__ __forceinline__ void run_group(const T *base, const int j, const int c0, const Taps &tp, float2 (&W)[NO][3][2]) {
+  constexpr int SK = C::EJ * C::EI, SJ = C::EI;
+  static_assert(27 <= TAP_PAIRS, "coefficient pairs");
+  const unsigned sb = smem_u32(base);
+#pragma unroll
+  for (int q = 0; q < 2 + NO; ++q) {  // tile plane k0 + q: brick-local plane k0 - 1 + q
+    float2 v[3][2];
+#pragma unroll
+    for (int rr = 0; rr < 3; ++rr)
+      ld_quad((T *)nullptr, sb + (unsigned)((q * SK + rr * SJ + C::col(j + rr, c0)) * (int)sizeof(T)), v[rr][0], v[rr][1]);
+#pragma unroll
+    for (int o = 0; o < NO; ++o) {
+      const int dk = q - o;  // 0, 1, 2: planes k - 1, k, k + 1 of row k0 + o
+      if (dk < 0 || dk > 2) continue;
+#pragma unroll
+      for (int rr = 0; rr < 3; ++rr)
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float2 c = tp.cp[(dk * 3 + rr) * 3 + d];
+            W[o][d][h] = dk == 0 && rr == 0 ? __fmul2_rn(c, v[rr][h]) : __ffma2_rn(c, v[rr][h], W[o][d][h]);
+          }
+    }
+  }
+}
+
+// The window after group W: the outputs it starts, and W_-1 of its last column.
+template <int NO>
+__device__ __forceinline__ void run_next(RunWin<NO> &S, const float2 (&W)[NO][3][2]) {
+#pragma unroll
+  for (int o = 0; o < NO; ++o) {
+    S.part[o][0] = (S.last[o] + W[o][1][0].x) + W[o][2][0].y;
+    S.part[o][1] = (W[o][0][0].x + W[o][1][0].y) + W[o][2][1].x;
+    S.part[o][2] = (W[o][0][0].y + W[o][1][1].x) + W[o][2][1].y;
+    S.part[o][3] = W[o][0][1].x + W[o][1][1].y;
+    S.last[o] = W[o][0][1].y;
+  }
+}
+
+// A brick's eight outputs of each row, parked from tile column c0 on and written.
+template <typename C, typename T, int NO>
+__device__ __forceinline__ void run_write(T *rt, T *ob, const int lane, const int c0, const RunWin<NO> &S) {
+  constexpr int SK = C::EJ * C::EI, SJ = C::EI;
+  const int k0 = NO * (lane >> 3), j = lane & 7;
+  T *park = rt + (k0 + 1) * SK + (j + 1) * SJ;
+  __syncwarp();  // every lane is past its reads of these columns
+#pragma unroll
+  for (int o = 0; o < NO; ++o) {
+    sts_quad((T *)nullptr, smem_u32(park + o * SK + C::col(j + 1, c0)), S.head[o]);
+    sts_quad((T *)nullptr, smem_u32(park + o * SK + C::col(j + 1, c0 + 4)), S.part[o]);
+  }
+  __syncwarp();  // the parked outputs of every lane are in the tile
+  cs_store<C, 1>(rt, ob, lane, c0);
+}
+
+// One brick (ob: its output): lo: the stream continues into it, so the brick before (pending) is
+// written here; more: the stream goes on into the next brick, which writes this one.  FP32 writes
+// the brick before as soon as it is complete, out of the first group's columns and the i-lo ones,
+// not fetched then (fewer registers: 291 us against 310); BF16 after the second group, whose loads
+// need not wait for it (241 us against 250).
+template <typename C, typename T>
+__device__ __forceinline__ void cube_istream4(T *rt, T *ob, T *&pending, const int lane, const Taps &tp,
+                                              RunWin<C::CSROWS> &S, const bool lo, const bool more) {
+  constexpr int SK = C::EJ * C::EI, SJ = C::EI, RP = C::RP, NO = C::CSROWS;
+  static_assert(C::TPB == 32 && NO == 2 && RP >= 4 && C::NEED >= RP + 12, "one warp, two rows per lane");
+  const int k0 = NO * (lane >> 3), j = lane & 7;
+  const T *base = rt + k0 * SK + j * SJ;
+  float2 W[NO][3][2];
+  if (!lo) run_edge<C, T, NO, 0>(base, j, RP - 1, tp, S.last);
+  run_group<C, T, NO>(base, j, RP, tp, W);
+  constexpr bool EARLY = sizeof(T) == 4;
+  RunWin<NO> before;
+  if (lo) {
+#pragma unroll
+    for (int o = 0; o < NO; ++o) S.part[o][3] += W[o][2][0].x;
+    if constexpr (EARLY) run_write<C, T, NO>(rt, pending, lane, RP - 4, S);
+    else before = S;
+  }
+  run_next<NO>(S, W);
+  run_group<C, T, NO>(base, j, RP + 4, tp, W);
+#pragma unroll
+  for (int o = 0; o < NO; ++o) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t) S.head[o][t] = S.part[o][t];
+    S.head[o][3] += W[o][2][0].x;
+  }
+  run_next<NO>(S, W);
+  if (!EARLY && lo) run_write<C, T, NO>(rt, pending, lane, RP, before);
+  pending = ob;
+  if (!more) {
+    float w[NO];
+    run_edge<C, T, NO, 2>(base, j, RP + 8, tp, w);
+#pragma unroll
+    for (int o = 0; o < NO; ++o) S.part[o][3] += w[o];
+    run_write<C, T, NO>(rt, ob, lane, RP, S);
   }
 }
 
@@ -925,8 +1071,7 @@ __device__ __forceinline__ void sweep2_brick(const T *rt, T *out_brick, int lt, 
   if constexpr (C::PAIR) {
     // lane -> (row, column pair); 16-byte pairs: rows 0,2,1,3 per quarter warp, two rows apart
     const int q = lt >> 2, i0 = 2 * (lt & 3);
-    // (rows of 12 words: the even rows' pairs fall in different banks, and the odd rows')
-    const int jp = C::PERM ? (q & 4) | ((q & 1) << 1) | ((q >> 1) & 1) : C::HALO4 ? ((q & 3) << 1) | (q >> 2) : q;
+    const int jp = C::PERM ? (q & 4) | ((q & 1) << 1) | ((q >> 1) & 1) : q;
     if constexpr (C::ES == 8)
       sym_cube_pair_shared<C, T, R, FAM == FAM_CUBESYM_IJ>(rt, out_brick + (size_t)(jp * BI + i0), jp, i0, tp);
     else
@@ -1320,8 +1465,9 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
   typedef Sweep2Cfg<T, BK, BJ, BI, R, FAM, ACC, IST> C;
   constexpr int TPB = C::TPB, NB = C::NB, EPT = C::EPT;
   static_assert(!IST || (C::ES == 8 && C::PAIR && NB == 1 && (FAM == FAM_CUBESYM || FAM == FAM_CUBESYM_IJ)) ||
-                    (C::ES <= 4 && C::CS4 && NB == 1 && FAM == FAM_CUBESYM && ACC != ACCM_FF),
-                "class-sum streams: mirror-symmetric cubes, FP64 (native) or FP32 / BF16 storage, one brick per CTA");
+                    (C::ES <= 4 && C::CS4 && NB == 1 && ACC != ACCM_FF &&
+                     (FAM == FAM_CUBESYM || (FAM == FAM_CUBE && R == 1 && ACC == ACCM_NATIVE))),
+                "streams: mirror-symmetric cubes, FP64 (native) or FP32 / BF16 storage, and the radius-1 cube on the latter");
   // streams run along the list, plain or batch mode (in batch mode a stream continues only
   // within one domain's field)
   constexpr bool STREAM = IST;
@@ -1338,7 +1484,7 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
 #pragma unroll
   for (int e = 0; e < EPT; ++e) {
     const int g = e * TPB + lt;
-    plan[e] = g < C::NV ? plan_entry<C, BK, BJ, BI, R, FAM, IST>(g) : 0u;
+    plan[e] = C::DEFER || g < C::NV ? plan_entry<C, BK, BJ, BI, R, FAM, IST>(g) : 0u;
   }
 
   const long long ngroups = ((long long)a.nlist + NB - 1) / NB;
@@ -1361,7 +1507,7 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
   // a position in this CTA's walk: the group and, chunked, its place in its chunk
   struct Walk {
     long long g;
-    long long pos;
+    int pos;
   };
   auto advance = [&](Walk w) -> Walk {
     if constexpr (CHUNKED) return w.pos + 1 < CH ? Walk{w.g + 1, w.pos + 1} : Walk{w.g + 1 + (G - 1) * CH, 0};
@@ -1378,73 +1524,77 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
   // entry, the adjacency and the checks in one place, a brick's warps stood still for two trips to
   // memory: GB300, 512^3, FP32 cube125 519 -> 494 us, FP64 2272 -> 2238, BF16 cube27 326 -> 314.
   constexpr int APT = (27 + TPB - 1) / TPB;  // adjacency entries per thread
-  uint2 ent = make_uint2(0, 0);              // batch: domain, brick; plain: -, brick
-  unsigned av[APT];
-  bool alive = false, listed = false;  // the group has an entry here; its brick is in range
-  long long achunks = 0;               // batch: bricks of the domain's fields
-  // batch: the domain's fields and their bytes per brick
-  const unsigned char *fin = nullptr;
-  unsigned char *fout = nullptr;
-  unsigned long long fstep = 0;
-  auto fetch_entry = [&](long long grp) {
-    const long long n = grp * NB + slot;
-    if (grp < gend && n < a.nlist) {
-      if constexpr (BATCH) ent = a.work[n];
-      else ent.y = a.blist[n];
-    }
+  struct Fetched {
+    unsigned av[APT];
+    bool alive, listed;  // the group has an entry here; its brick is in range
+    // batch: the bricks of the domain's fields, the fields, their bytes per brick
+    long long chunks;
+    const unsigned char *fin;
+    unsigned char *fout;
+    unsigned long long fstep;
   };
-  auto fetch_adj = [&](long long grp) {
+  auto fetch_entry = [&](long long grp) -> uint2 {  // batch: domain, brick; plain: -, brick
     const long long n = grp * NB + slot;
-    alive = grp < gend && n < a.nlist;
-    listed = false;
-    if (!alive) return;
+    uint2 e = make_uint2(0, 0);
+    if (grp < gend && n < a.nlist) {
+      if constexpr (BATCH) e = a.work[n];
+      else e.y = a.blist[n];
+    }
+    return e;
+  };
+  auto fetch_adj = [&](long long grp, uint2 ent) -> Fetched {
+    const long long n = grp * NB + slot;
+    Fetched f{};
+    f.alive = grp < gend && n < a.nlist;
+    if (!f.alive) return f;
     const unsigned *adj = a.adj;
     if constexpr (BATCH) {
       const bool dok = ent.x < a.ndom;
       const BatchDomain &D = a.doms[dok ? ent.x : 0];
       adj = D.adj;
-      achunks = D.chunks;
-      listed = dok && ent.y < D.nbricks;
-      fin = reinterpret_cast<const unsigned char *>(a.parity ? D.f1 : D.f0);
-      fout = reinterpret_cast<unsigned char *>(a.parity ? D.f0 : D.f1);
-      fstep = D.step_bytes;
+      f.chunks = D.chunks;
+      f.listed = dok && ent.y < D.nbricks;
+      f.fin = reinterpret_cast<const unsigned char *>(a.parity ? D.f1 : D.f0);
+      f.fout = reinterpret_cast<unsigned char *>(a.parity ? D.f0 : D.f1);
+      f.fstep = D.step_bytes;
     } else {
-      listed = ent.y < a.nbricks;
+      f.listed = ent.y < a.nbricks;
     }
-    if (listed) {
+    if (f.listed) {
 #pragma unroll
       for (int q = 0; q < APT; ++q) {
         const int sl = lt + q * TPB;
-        if (sl < 27) av[q] = adj[(size_t)ent.y * 27 + sl];
+        if (sl < 27) f.av[q] = adj[(size_t)ent.y * 27 + sl];
       }
     }
+    return f;
   };
-  auto store_adj = [&](int ns) {
+  auto store_adj = [&](int ns, const Fetched &f) {
     Staged &nb = nbrs[ns * NB + slot];
-    const long long in_chunks = BATCH ? achunks : a.in_chunks, out_chunks = BATCH ? achunks : a.out_chunks;
+    const long long in_chunks = BATCH ? f.chunks : a.in_chunks, out_chunks = BATCH ? f.chunks : a.out_chunks;
     const unsigned char *in =
-        BATCH ? fin : reinterpret_cast<const unsigned char *>(reinterpret_cast<const T *>(a.in) + a.in_off);
-    const size_t in_step = BATCH ? fstep : a.in_step * sizeof(T);
+        BATCH ? f.fin : reinterpret_cast<const unsigned char *>(reinterpret_cast<const T *>(a.in) + a.in_off);
+    const size_t in_step = BATCH ? f.fstep : a.in_step * sizeof(T);
 #pragma unroll
     for (int q = 0; q < APT; ++q) {
       const int sl = lt + q * TPB;
       if (sl < 27) {
-        unsigned v = listed ? av[q] : 0u;
-        bool ok = listed;
-        if (listed) {
+        unsigned v = f.listed ? f.av[q] : 0u;
+        bool ok = f.listed;
+        if (f.listed) {
           if (sl == 13 && (long long)v >= out_chunks) ok = false;
           if ((long long)v >= in_chunks) ok = false;
           if (!ok) {  // a neighbour out of range reads brick 0, a centre out of range does not run
             atomicOr(a.err, FLAG_BOUNDS);
             v = 0;
           }
-        } else if (alive && sl == 13) {
+        } else if (f.alive && sl == 13) {
           atomicOr(a.err, FLAG_BOUNDS);
         }
         nb.src[sl] = in + v * in_step;
         if (sl == 13) {
           nb.active = ok;
-          nb.out = BATCH ? fout + v * fstep
+          nb.out = BATCH ? f.fout + v * f.fstep
                          : reinterpret_cast<unsigned char *>(reinterpret_cast<T *>(a.out) + a.out_off + v * a.out_step);
         }
       }
@@ -1471,35 +1621,51 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
   // come from the previous brick), so copies wholly before ICUT are skipped
   // plan entries a continued brick issues: those of the first NVN copies (warp-uniform bound)
   constexpr int EPTN = STREAM ? (StreamPlan<C, R>::NVN + TPB - 1) / TPB : EPT;
-  // copies [E0, E1) of this thread: the neighbours' addresses are read from shared memory ISSUE
-  // copies at a time, ahead of the copies, which the compiler keeps in order with every access (a
-  // brick index read and multiplied out in front of each copy: GB300, 512^3, FP32 cube125 494 us
-  // against 454, FP64 2238 against 2161, BF16 424 against 378)
-  auto copies = [&](auto first, auto last, const Staged &nb, unsigned tbase) {
-    constexpr int E0 = decltype(first)::value, E1 = decltype(last)::value, STEP = C::ISSUE;
+  // copies [E0, E1) of this thread, the first N over the brick's threads.  The neighbours' addresses
+  // are read from shared memory ISSUE copies at a time, ahead of the copies, which the compiler
+  // keeps in order with every access (a brick index read and multiplied out in front of each copy:
+  // GB300, 512^3, FP32 cube125 494 us against 454, FP64 2238 against 2161, BF16 424 against 378)
+  auto copies = [&](auto first, auto last, auto number, const Staged &nb, unsigned tbase, auto hi) {
+    constexpr int E0 = decltype(first)::value, E1 = decltype(last)::value, N = decltype(number)::value, STEP = C::ISSUE;
+    // an i-hi copy from its i-lo twin: two slots on, the brick's first columns, the tile row's last
+    auto entry = [&](int e) -> unsigned {
+      if (!decltype(hi)::value) return plan[e];
+      const unsigned p = plan[e] + 2u - ((unsigned)((BI - C::RP) % BI) << 5);
+      return C::SWZ ? p ^ ((unsigned)(C::RP + BI) << 18) : p + ((unsigned)(C::RP + BI) << 18);
+    };
 #pragma unroll
     for (int e0 = E0; e0 < E1; e0 += STEP) {
       const unsigned char *g[STEP];
 #pragma unroll
       for (int x = 0; x < STEP; ++x)
-        if (e0 + x < E1) g[x] = nb.src[plan[e0 + x] & 31u] + ((plan[e0 + x] >> 5) & 8191u) * (unsigned)C::ES;
+        if (e0 + x < E1) g[x] = nb.src[entry(e0 + x) & 31u] + ((entry(e0 + x) >> 5) & 8191u) * (unsigned)C::ES;
 #pragma unroll
       for (int x = 0; x < STEP; ++x) {
         const int e = e0 + x;
-        if (e < E1 && e * TPB + lt < (E1 == EPT ? C::NV : StreamPlan<C, R>::NVN)) {
-          const unsigned dst = tbase + (plan[e] >> 18) * (unsigned)C::ES;
-          if (C::HALO4 && e * TPB + lt >= C::NV_ROWS) cp_async<4>(dst, g[x]);
-          else cp_async<C::VB>(dst, g[x]);
+        if (e < E1 && (e - E0) * TPB + lt < N) {
+          const unsigned dst = tbase + (entry(e) >> 18) * (unsigned)C::ES;
+          cp_async<C::VB>(dst, g[x]);
         }
       }
     }
   };
-  auto issue = [&](int buf, int ns, bool cont) {
+  // lo: the stream continues into this brick; hi (DEFER): and from it into the next
+  auto issue = [&](int buf, int ns, bool lo, bool hi) {
     const Staged &nb = nbrs[ns * NB + slot];
     if (nb.active) {
       const unsigned tbase = smem_u32((buf ? raw1 : raw0) + slot * C::TILE_BYTES);
-      if (STREAM && cont) copies(Int<0>{}, Int<EPTN>{}, nb, tbase);
-      else copies(Int<0>{}, Int<EPT>{}, nb, tbase);
+      constexpr Int<0> NOT{};
+      if constexpr (C::DEFER) {
+        constexpr Int<C::EPT_MID> M{};
+        copies(Int<0>{}, M, Int<C::NV_MID>{}, nb, tbase, NOT);
+        if (!lo) copies(M, Int<EPT>{}, Int<C::NV_SIDE>{}, nb, tbase, NOT);
+        if (!hi) copies(M, Int<EPT>{}, Int<C::NV_SIDE>{}, nb, tbase, Int<1>{});
+      } else if constexpr (STREAM) {
+        if (lo) copies(Int<0>{}, Int<EPTN>{}, Int<StreamPlan<C, R>::NVN>{}, nb, tbase, NOT);
+        else copies(Int<0>{}, Int<EPT>{}, Int<C::NV>{}, nb, tbase, NOT);
+      } else {
+        copies(Int<0>{}, Int<EPT>{}, Int<C::NV>{}, nb, tbase, NOT);
+      }
     }
     cp_async_commit();
   };
@@ -1520,37 +1686,48 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
                 "fixed point: stars and cubes on 8x8x8 bricks, 64 threads each");
 
   grid_begin();
-  // prologue: adjacency of the first two groups, copies of the first
-  Walk w1{g0, 0};
-  Walk w2 = advance(w1), w3 = advance(w2);  // the next group and the one after
-  long long grp = g0;
-  fetch_entry(grp);
-  fetch_adj(grp);
-  fetch_entry(w2.g);
-  store_adj(0);
-  fetch_adj(w2.g);
-  fetch_entry(w3.g);
-  store_adj(1);
+  // prologue: adjacency of the first groups, copies of the first
+  constexpr int AHEAD = C::DEFER ? 3 : 2;  // groups staged ahead (DEFER: the current one's slot is free)
+  const Walk w1 = advance(Walk{g0, 0}), w2 = advance(w1);
+  long long grp = g0, grp1 = w1.g, grp2 = w2.g;  // the current group, the next, the one after
+  Walk far = C::DEFER ? advance(w2) : w2;        // the one to stage
+  uint2 ent;
+  {  // every load before the first is waited for: the entries, then the adjacencies
+    const uint2 e0 = fetch_entry(grp), e1 = fetch_entry(grp1), e2 = fetch_entry(grp2);
+    ent = C::DEFER ? fetch_entry(far.g) : e2;
+    const Fetched f0 = fetch_adj(grp, e0), f1 = fetch_adj(grp1, e1);
+    Fetched f2;
+    if constexpr (C::DEFER) f2 = fetch_adj(grp2, e2);
+    store_adj(0, f0);
+    store_adj(1, f1);
+    if constexpr (C::DEFER) store_adj(2, f2);
+  }
   __syncthreads();
-  issue(0, 0, false);
+  // DEFER: the stream continues into the current group; from it into the next; the brick before it
+  // is still to be written; its own output brick; it runs
+  bool lo = false, more = C::DEFER && continues(0, 1), runs = nbrs[slot].active != 0;
+  T *pending = nullptr, *obrick = reinterpret_cast<T *>(nbrs[slot].out);
+  issue(0, 0, false, more);
 
   // i-streaming: W of the last 2R columns of the previous brick (sym_cube_istream), or of the
   // last two 4-column groups (sym_cube_istream4)
   double W[IST && C::ES == 8 ? 2 : 1][IST && C::ES == 8 ? R + 1 : 1][IST && C::ES == 8 ? 2 * R + 1 : 1];
   CsWin<R, ACC == ACCM_COMP, C::CSROWS> S4;
+  RunWin<C::CSROWS> run{};  // cube_istream4
 
-  for (int it = 0; grp < gend; grp = w2.g, w2 = w3, w3 = advance(w3), ++it) {
+  for (int it = 0; grp < gend; ++it) {
     const int cur = it & 1, nxt = cur ^ 1;
-    const int ncur = it % 3, nnxt = (it + 1) % 3, nfar = (it + 2) % 3;
+    const int ncur = it % 3, nnxt = (it + 1) % 3, nfar = (it + AHEAD) % 3;
     __syncthreads();     // nbrs[nnxt] visible; every thread is done with raw[nxt] and nbrs[nfar]
-    issue(nxt, nnxt, STREAM && continues(ncur, nnxt));
-    fetch_adj(w3.g);             // lands while this group computes
-    fetch_entry(advance(w3).g);  // lands by the next group's turn
+    const bool hi = C::DEFER && continues(nnxt, (it + 2) % 3);
+    issue(nxt, nnxt, C::DEFER ? more : STREAM && continues(ncur, nnxt), hi);
+    const Fetched f = fetch_adj(far.g, ent);  // lands while this group computes
+    ent = fetch_entry(advance(far).g);        // lands by the next group's turn
     cp_async_wait<1>();  // this thread's copies for the current group have landed
     __syncthreads();     // ... and everybody else's
 
     const Staged &nbr = nbrs[ncur * NB + slot];
-    const bool active = nbr.active != 0;
+    const bool active = C::DEFER ? runs : nbr.active != 0;
     const T *rt = reinterpret_cast<const T *>((cur ? raw1 : raw0) + slot * C::TILE_BYTES);
     if constexpr (ACC == ACCM_FF) {
       // one pass, in place: raw doubles -> float pairs (each thread its own elements)
@@ -1565,13 +1742,15 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
       // and centre columns
       // (the same test the gather of this group was issued with: its skipped columns are the
       // ones a continued stream does not read)
-      const bool cont = STREAM && it > 0 && continues(nfar, ncur);
+      const bool cont = C::DEFER ? lo : it > 0 && continues(nfar, ncur);
       if (active) {
-        T *ob = reinterpret_cast<T *>(nbr.out);
+        T *ob = C::DEFER ? obrick : reinterpret_cast<T *>(nbr.out);
         T *tile = const_cast<T *>(rt);  // this brick's buffer until the next barrier
         if constexpr (C::ES == 8) {
           if (tp.kj) sym_cube_istream<C, R, true>(tile, ob, lt, tp, W, cont);
           else sym_cube_istream<C, R, false>(tile, ob, lt, tp, W, cont);
+        } else if constexpr (FAM == FAM_CUBE) {
+          cube_istream4<C, T>(tile, ob, pending, lt, tp, run, cont, more);
         } else {
           constexpr bool CM = ACC == ACCM_COMP;
           if (tp.kj) sym_cube_istream4<C, T, R, true, CM>(tile, ob, lt, tp, S4, cont);
@@ -1593,7 +1772,17 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
       } else
         sweep2_brick<T, BK, BJ, BI, R, FAM, ACC>(rt, ob, lt, tp, cs);
     }
-    store_adj(nfar);  // group it + 2; read after the next iteration's first barrier
+    store_adj(nfar, f);  // group it + AHEAD; read after the next iteration's first barrier
+    if constexpr (C::DEFER) {
+      lo = more;
+      more = hi;
+      runs = nbrs[nnxt * NB + slot].active != 0;
+      obrick = reinterpret_cast<T *>(nbrs[nnxt * NB + slot].out);
+    }
+    grp = grp1;
+    grp1 = C::DEFER ? grp2 : far.g;
+    grp2 = far.g;
+    far = advance(far);
   }
   cp_async_wait<0>();  // no copy may outlive the kernel
 }
