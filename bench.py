@@ -249,9 +249,12 @@ def run_ours(args):
                             "pipe_frac": round(points / (dom_ms * 1e-3) * instr / (fp64_rate.value / 2), 4),
                             "note": "achieved counts 2 x taps flop per point; pipe_frac counts the floating-point "
                                     "instructions the kernel executes per point (mirror-symmetric cubes run on "
-                                    "pair sums) against the measured FMA instruction rate"}}
+                                    "pair sums) against the measured FMA instruction rate; native FP64 sums that "
+                                    "run in 64-bit fixed point on the integer multipliers take the place of that "
+                                    "many FP64 instructions, and the fraction exceeds one"}}
     pipe_frac = roofline["compute"]["pipe_frac"]
-    roofline["binding"] = (("fp64 pipe" if dtype == _abi.BK_F64 and acc != _abi.BK_ACC_FLOATFLOAT else "fp32 pipe")
+    roofline["binding"] = ("integer multipliers" if dtype == _abi.BK_F64 and pipe_frac > 1.1 else
+                           ("fp64 pipe" if dtype == _abi.BK_F64 and acc != _abi.BK_ACC_FLOATFLOAT else "fp32 pipe")
                            if pipe_frac > roofline["frac"] else "hbm")
 
     # end to end through the public API, every result in host memory.  Per step: the input is

@@ -1,9 +1,10 @@
 // Pipelined brick sweep for row-major brick layouts (sweep_kernel covers the rest).
 //
-// Persistent CTAs walk the brick list in groups of NB bricks (every gridDim.x-th group; a
-// contiguous share of the list per CTA for the FP64 mirror-symmetric cubes streamed along i,
-// sym_cube_istream).  For every group:
-//   * the 27 adjacency entries of each brick are staged in shared memory;
+// Persistent CTAs walk the brick list in groups of NB bricks (every gridDim.x-th group; for the
+// cubes streamed along i chunks of consecutive groups, 4- and 2-byte storage, or a contiguous share
+// of the list per CTA, FP64 class sums).  For every group:
+//   * the addresses of each brick's 27 neighbours are staged in shared memory, from list entries
+//     loaded three groups ahead and adjacency loaded two ahead;
 //   * every thread issues its share of the group's gather as asynchronous global->shared
 //     copies (cp.async, 16 bytes where the layout allows) into one of two tile buffers,
 //     following a per-thread plan computed once at kernel start: each plan entry is one
@@ -16,7 +17,9 @@
 // sit in registers, so k-direction taps cost no shared-memory loads; star stencils read
 // the i / j taps from the tile, cube stencils walk the (2R+1)^2 columns (the 8x8x8 cube
 // paths: a column pair per lane, or, streamed along i, two rows per lane).  Float-float
-// mode converts the raw FP64 tile into float pairs in one pass before computing.
+// mode converts the raw FP64 tile into float pairs in one pass before computing.  The fixed-point
+// modes of FP64 stars and cubes (fx.cuh) convert the tile into integers in place, brick by brick,
+// or sum the brick in FP64.
 #pragma once
 
 #include "sweep_kernel.cuh"

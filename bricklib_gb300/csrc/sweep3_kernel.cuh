@@ -20,7 +20,9 @@
 //     post the stage's byte count and issue the copies (mbarrier "full");
 //   * the other warps are consumers: wait for "full", compute, arrive on "empty".  Every
 //     thread computes one (j, i) column of its brick: k taps from registers, i / j taps from
-//     shared memory, the region (centre or face) chosen per lane.
+//     shared memory, the region (centre or face) chosen per lane.  FP64 in fixed point (fx.cuh): the
+//     brick's threads convert its values into a tile of their own and each computes half the planes
+//     of a column pair from it, or, where the brick's values do not allow it, its column in FP64.
 // No block-wide barrier runs in the loop.  Every wait gives up after about a second, sets a
 // device error flag and stops the CTA (the producer then waits, again bounded, for its
 // copies still in flight).  Summation order is that of the pipelined kernel.
@@ -417,7 +419,8 @@ __device__ __forceinline__ void star_fx_consume(unsigned char *sm, const unsigne
 
 // Resident CTAs asked of the register allocator for the fixed-point stars (radius 1, 2 and 4: 96, 120
 // and 128 registers).  256^3, us, with one CTA less / these / one more: 7-point star with one ring
-// coefficient 80 / 76 / 81, 13-point 117 / 104 / 117, 25-point 237 / 174 / --.
+// coefficient 80 / 76 / 81, 13-point 117 / 104 / 117; the 25-point one, whose tile
+// holds no more than three, 154.
 constexpr int star_tma_minb(int r, int acc) {
   return acc == ACCM_FX || acc == ACCM_FXS ? (r == 1 ? 4 : 3) : 0;
 }

@@ -48,7 +48,10 @@ typedef enum bk_status {
 typedef enum bk_dtype { BK_F64 = 0, BK_F32 = 1, BK_BF16 = 2 } bk_dtype;
 
 /* Arithmetic of a sweep.
- * BK_ACC_NATIVE      accumulate in the storage type (FP32 for BF16 storage)
+ * BK_ACC_NATIVE      accumulate in the storage type (FP32 for BF16 storage); FP64 stars and cubes on
+ *                    row-major 8x8x8 bricks (and 4-D radius-1 stars) sum bricks whose values allow it
+ *                    in 64-bit fixed point, the sum rounded once: closer to the exact sum than the
+ *                    FP64 chain, zero sums are +0; the other bricks in FP64
  * BK_ACC_COMPENSATED FP32/BF16 storage: FP32 accumulation with Neumaier compensation
  * BK_ACC_FLOATFLOAT  FP64 storage: products and sums in float-float (pairs of FP32,
  *                    error-free transforms of Dekker 1971 / Knuth TwoSum), relative
@@ -157,8 +160,8 @@ int bk_stencil_check(const bk_stencil *st, const bk_layout *lay, int *radius, in
  * Four kernels implement it: two TMA-fed ones for 7/13/25-point stars on row-major 8x8x8
  * bricks with 16-byte aligned input (FP32 / BF16: runs of i-adjacent list entries share
  * their i-neighbour bricks; FP64: per-brick staging), a pipelined one (row-major layouts,
- * 16-byte aligned input; FP64 mirror-symmetric cubes carry per-column sums along runs of
- * i-adjacent list entries, so a list in grid order is fastest) and a one-shot one
+ * 16-byte aligned input; FP32 / BF16 cubes carry per-column sums along runs of i-adjacent
+ * list entries, so a list in grid order is fastest) and a one-shot one
  * (everything).  The FP32 / BF16 row kernel and the cube kernels on 8x8x8 bricks store
  * output pairs: they need every output brick to start on a two-element boundary, and
  * other output fields take per-element stores.  The environment variables
@@ -166,7 +169,8 @@ int bk_stencil_check(const bk_stencil *st, const bk_layout *lay, int *radius, in
  * parity tests); BK_TMA_ROW=0 selects per-brick staging for FP32 / BF16, BK_TMA_GROUP=0/1
  * turns the row kernel's grouped copies of full runs off/on, BK_TMA_STAGES (2..4) and
  * BK_TMA_IFACE (narrow / whole) tune the TMA-fed kernels, BK_SWEEP_ISTREAM=0 computes
- * FP64 mirror-symmetric cubes one brick at a time. */
+ * the cubes that are streamed along runs of bricks one brick at a time (FP64: and without
+ * fixed point where they are mirror-symmetric). */
 int bk_sweep(const unsigned *adj, unsigned nbricks, const bk_field *in, const bk_field *out,
              const unsigned *blist, unsigned nlist, const bk_stencil *st, const bk_layout *lay,
              int acc, void *stream);
