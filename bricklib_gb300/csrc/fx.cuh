@@ -27,7 +27,8 @@
 // 2^(E - 1022): cut values 2^-XB sum |c|, rounded coefficients n 2^(-1 - q), one or two roundings of half
 // a unit 2^(64 - q - XB), and 2^(31 - q - XB) sum |cl|.  It is then at most n 2^-53 max |c_t x_t|, the
 // a-priori bound of the chain's own rounding errors.  (Values that are all exact do not do instead:
-// where all but one of a point's values are zero, the chain is exact but for one rounding.)
+// where all but one of a point's values are zero, the chain is exact but for one rounding.)  Bricks
+// that are zero throughout need no sums either way.
 #pragma once
 
 #include "bk_common.cuh"
@@ -180,7 +181,7 @@ template <bool PAIR, bool SWAP, bool SUM, bool BOX, int XB, class From, class To
 struct FxShare {
   static constexpr int NV = 8 + 2 * From::NP + From::NS;
   // values kept in registers between the scan and the conversion, or loaded again
-  static constexpr bool HOLD = NV <= 20;
+  static constexpr bool HOLD = NV <= 20, STAR = !BOX;
   int lt;
   From from;
   To to;
@@ -590,7 +591,19 @@ __device__ __forceinline__ bool fx_prepare(const Share &sh, const double *from, 
   if (stopped || !on) return false;
   const FxScan s = fx_gather(slot);
   E = (int)(s.top >> 20);
-  if (!fx_ok(tab, s)) return false;
+  // a star on zeros, or numbers below 2^-1042: where all are zero, so are the sums, on any scale (256^3
+  // zeros, us, in FP64 / so: 7-point 197 / 89, 13-point 359 / 104, 25-point 689 / 162; the cubes
+  // write their zeros themselves, sweep2_kernel)
+  if (Share::STAR && s.top == 0) {
+    if constexpr (!Share::HOLD) sh.load(from, v);
+    bool some = false;
+#pragma unroll
+    for (int q = 0; q < Share::NV; ++q) some = some || __double2loint(v[q]) != 0;
+    if (fx_bar_or(brick, some)) return false;
+    E = tab.elo;
+  } else if (!fx_ok(tab, s)) {
+    return false;
+  }
   if constexpr (!Share::HOLD) sh.load(from, v);
   taken();
   sh.convert(to, v, E);

@@ -518,7 +518,7 @@ struct SweepPlan {
   bool symij; // ... and symmetric under the i <-> j swap
   bool ops;   // pointwise pre / post operations (one-shot kernels only)
   bool out_pair;  // every output brick starts on a boundary of two elements (pair stores)
-  bool istream;   // FP64 mirror-symmetric 8x8x8 cubes: columns streamed along i
+  bool istream;   // 8x8x8 cubes whose column sums may be streamed along i (plan_sweep)
   int fam;
   int r;
   int acc;

@@ -89,6 +89,25 @@ def test_fixed_point_sweeps_against_the_oracle(name, kind):
     check(dom, arr, st, dom.interior_view(dom.get_field(1)))
 
 
+@pytest.mark.parametrize("name", STENCILS)
+def test_fixed_point_zero_bricks(name):
+    """Bricks whose values are all zero (of either sign) are not summed; denormals beside zeros are."""
+    st = stencil(name)
+    dom = GridDomain((24, 32, 40), dtype=BK_F64)
+    arr, o = np.zeros(dom.adims), dom.org
+    arr[o[0]:o[0] + 8, o[1]:o[1] + 12] = -0.0
+    arr[o[0] + 16:o[0] + 24, o[1] + 8:o[1] + 16, o[2] + 8:o[2] + 16] = 1e-320
+    arr[o[0] + 8, o[1] + 24, o[2] + 24] = 1e-318  # a corner of one brick, in the reach of its neighbours
+    arr[o[0] + 12:o[0] + 14, o[1] + 3, o[2] + 30:] = 0.75
+    dom.set_field(0, arr)
+    dom.upload()
+    B.brickSweep(dom.brick(0), dom.brick(1), dom.dev_interior, st)
+    B.synchronize()
+    assert B.error_flags() == 0
+    dom.download()
+    check(dom, arr, st, dom.interior_view(dom.get_field(1)))
+
+
 @pytest.mark.parametrize("name", ["star7", "star13", "star25", "cube27", "cube125"])
 @pytest.mark.parametrize("count,off", [(1, 0), (7, 0), (60, 1)])
 def test_fixed_point_short_lists_and_odd_output_fields(name, count, off):
