@@ -1471,8 +1471,8 @@ __device__ __forceinline__ auto sweep2_share(int lt) {
   }
 }
 
-// IST: FP64 mirror-symmetric cubes streamed along i (sym_cube_istream): each CTA takes a
-// contiguous share of the list instead of every gridDim.x-th group.
+// IST: cubes streamed along i: each CTA takes a contiguous share of the list (FP64) or chunks of
+// consecutive groups (4- and 2-byte storage) instead of every gridDim.x-th group.
 template <typename T, int BK, int BJ, int BI, int R, int FAM, int ACC, bool BATCH, bool IST>
 __global__ void __launch_bounds__(Sweep2Cfg<T, BK, BJ, BI, R, FAM, ACC, IST>::NT,
                                   Sweep2Cfg<T, BK, BJ, BI, R, FAM, ACC, IST>::MINB)
