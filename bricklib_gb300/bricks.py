@@ -186,8 +186,12 @@ class Layout:
         return int(np.prod(self.bdim))
 
     def to_c(self) -> _abi.bk_layout:
-        # packed rather than assigned member by member: each sweep makes one (2.7 against 0.9 us)
-        return _abi.bk_layout.from_buffer_copy(_PACK3(*self.bdim) + _PACK3(*self.fold))
+        # packed rather than assigned member by member: each sweep makes one (2.7 against 0.9 us);
+        # ctypes says what becomes of whatever does not pack
+        try:
+            return _abi.bk_layout.from_buffer_copy(_PACK3(*self.bdim) + _PACK3(*self.fold))
+        except struct.error:
+            return _abi.bk_layout((C.c_int * 3)(*self.bdim), (C.c_int * 3)(*self.fold))
 
     def offsets(self) -> np.ndarray:
         """layout(k, j, i) for every element in row-major (k, j, i) order
