@@ -34,19 +34,19 @@ static int shape_of(const Layout &L) {
 // 4 k; near[0]: the centre), whose terms are checked; the products multiply `slots` sums, sum s of
 // count[s] values with coefficient c[first[s]].  Left off (false) for coefficients so uneven that many
 // bricks of ordinary values would fail the check and run in FP64, and for stencils whose
-// coefficients after the first are all powers of two (the 7-point Laplacian): their products are
+// coefficients but the centre's are all powers of two (the 7-point Laplacian): their products are
 // exact, so the FP64 chain rounds exactly as the reference's CPU code does, which callers that
 // compare cancelling sums with it rely on.
 bool fx_table(const double *c, int n, const int (*near)[9], int masks, int slots, const int *first, const int *count,
               int xb, bool one, FxTab *t) {
   t->on = 0;
   double sum = 0.0, most = 0.0, heads = 0.0;
-  bool exact = true;  // c[k] x exact for every k > 0
+  bool exact = true;  // c[k] x exact for every k but the centre
   for (int k = 0; k < n; ++k) {
     sum += fabs(c[k]);
     most = fmax(most, fabs(c[k]));
     int e;
-    if (k && c[k] != 0.0) exact = exact && fabs(frexp(c[k], &e)) == 0.5;
+    if (k != near[0][0] && c[k] != 0.0) exact = exact && fabs(frexp(c[k], &e)) == 0.5;
   }
   if (exact || !(sum > 1e-270) || !(sum < 1e270)) return false;
   for (int s = 0; s < slots; ++s) heads += fabs(c[first[s]]);
