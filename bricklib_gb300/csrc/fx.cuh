@@ -16,19 +16,23 @@
 // whose first three sums are exact 64-bit integers and whose last (below 2^-61 of the largest total
 // per product, with no preferred sign) is left out.  The total is rounded to units of 2^64 (2^-59
 // of the largest possible one, less where values are added before they are multiplied) and then
-// to a double.  Integer sums do not depend on their
-// order: every kernel gives the same bits.
+// to a double.  Integer sums do not depend on their order: every kernel that sums a brick this way
+// gives the same bits.
 //
-// A brick is computed this way only when the result is at least as good as the chain of n FP64
-// multiply-adds would give, else its threads run that chain: E within the range where results
+// A brick is computed this way only when the error bound is no larger than that of the chain of n
+// FP64 multiply-adds, else its threads run FP64: E within the range where results
 // are normal numbers (which leaves out infinities and NaNs), and every point has a term
 // |c_t x_t| >= error / (n 2^-53) among its centre tap and, within its 2 x 2 x 2 block, its neighbour on
 // each axis (cubes: all seven others).  error is the bound of what goes wrong here, in units of
 // 2^(E - 1022): cut values 2^-XB sum |c|, rounded coefficients n 2^(-1 - q), one or two roundings of half
 // a unit 2^(64 - q - XB), and 2^(31 - q - XB) sum |cl|.  It is then at most n 2^-53 max |c_t x_t|, the
-// a-priori bound of the chain's own rounding errors.  (Values that are all exact do not do instead:
-// where all but one of a point's values are zero, the chain is exact but for one rounding.)  Bricks
-// that are zero throughout need no sums either way.
+// a-priori bound of the chain's own rounding errors; the rounding of the total to a double, half a
+// unit of the result's last place, comes on top.  On uniform values the result is closer to the
+// exact sum than the chain's; it need not be where a point has one large term and the others are
+// next to nothing, since the chain then rounds once (half a unit of 2^-53; 1.07 of them were found
+// here for a 7-point heat step on isolated values beside one 2^5 as large).  (Values that are all exact
+// do not do instead of the check: where all but one of a point's values are zero, the chain is exact
+// but for one rounding.)  Bricks that are zero throughout need no sums either way.
 #pragma once
 
 #include "bk_common.cuh"

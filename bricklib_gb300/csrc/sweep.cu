@@ -75,11 +75,14 @@ bool fx_table(const double *c, int n, const int (*near)[9], int masks, int slots
     if (fits) break;
   }
   if (!fits) return false;
-  // weights of the checked terms: a term c x passes when the high words of x and of
-  // c / (2 error / (n 2^-53)), added as exponents with fractions, reach exponent E (the sum of two
-  // high words never exceeds the high word of the product, so this errs towards FP64).  error: of
-  // the sum made here, in units of 2^(E - 1022): cut values, rounded coefficients, one or two
-  // roundings of half a unit (one: FxAcc<true>), sum cl xl
+  // weights of the checked terms: a term c x passes when the high words of x and c less that of
+  // least = 2 error / (n 2^-53), as exponents with fractions, reach exponent E.  That never lets a
+  // term below the bound through: with mantissas in [1, 2), l that of least and d >= 0 its distance
+  // from c's, the smallest x that reaches the octave has c x / least = 2^(E - 1023) times
+  // 1 + d (2 - l - d) / (2 l) where c's is the larger (d < 2 - l), 1 + d (l - 1 - d) / l where least's
+  // is (d <= l - 1).  error: of the sum made here, in units of
+  // 2^(E - 1022): cut values, rounded coefficients, one or two roundings of half a unit (one:
+  // FxAcc<true>), products cl xl left out
   const double error = ldexp(sum, -xb) + ldexp((double)n, -1 - t->q) + ldexp(one ? 0.5 : 1.0, 64 - t->q - xb) + ldexp(low, 31 - t->q - xb);
   const double least = 2.0 * error / (n * ldexp(1.0, -53));
   double bits = 0.0;
