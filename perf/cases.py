@@ -313,7 +313,7 @@ def run_move(s):
     inner = [n[2], n[1], n[0]]
     whole = [n[2] + 2 * gh[2], n[1] + 2 * gh[1], n[0] + 2 * gh[0]]
     g = [gh[2], gh[1], gh[0]]
-    B.copyToBrickDevice(inner, g, g, s["arr"].data_ptr(), s["grid_dev"].ptr, s["a"])
+    B.copyToBrickDevice(inner, [0, 0, 0], g, s["arr"].data_ptr(), s["grid_dev"].ptr, s["a"])
     B.ghostFill(s["plan"], s["a"])
     B.copyFromBrickDevice(whole, [0, 0, 0], [0, 0, 0], s["back"].data_ptr(), s["grid_dev"].ptr, s["a"])
     return s["ta"], s["back"]
