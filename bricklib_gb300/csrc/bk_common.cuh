@@ -38,7 +38,8 @@ constexpr int FLAG_TIMEOUT = 2;
 template <class... P, class... A>
 cudaError_t launch_overlapped(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, const A &...args) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  const bool eager = cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+  const cudaError_t asked = cudaStreamIsCapturing(s, &cap);
+  const bool eager = asked == cudaSuccess && cap == cudaStreamCaptureStatusNone;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -49,7 +50,10 @@ cudaError_t launch_overlapped(void (*kern)(P...), unsigned grid, unsigned thread
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = eager ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P(args)...);
+  // the caller has the error: it is not left as the thread's last one, by which plain launches are checked
+  if (asked != cudaSuccess || e != cudaSuccess) (void)cudaGetLastError();
+  return e;
 }
 
 // The CTAs of `threads` threads and `smem` bytes of dynamic shared memory that the current device
