@@ -50,26 +50,30 @@ int kernel_fit(const void *kern, int threads, size_t smem, int *sms, int *per_sm
   struct Fit {
     int sms, per_sm;
   };
-  static std::mutex mu;
-  static std::map<std::tuple<const void *, int, int, size_t>, Fit> fits;
-  static std::map<std::pair<const void *, int>, size_t> allowed;  // the attribute as last raised
+  // never destroyed: a server's thread may launch while the process ends
+  struct Tables {
+    std::mutex mu;
+    std::map<std::tuple<const void *, int, int, size_t>, Fit> fits;
+    std::map<std::pair<const void *, int>, size_t> allowed;  // the attribute as last raised
+  };
+  static Tables &t = *new Tables;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(e, what);
-  std::lock_guard<std::mutex> lk(mu);
+  std::lock_guard<std::mutex> lk(t.mu);
   const auto key = std::make_tuple(kern, dev, threads, smem);
-  auto it = fits.find(key);
-  if (it == fits.end()) {
+  auto it = t.fits.find(key);
+  if (it == t.fits.end()) {
     Fit f{0, 0};
     e = cudaDeviceGetAttribute(&f.sms, cudaDevAttrMultiProcessorCount, dev);
-    size_t &most = allowed[{kern, dev}];
+    size_t &most = t.allowed[{kern, dev}];
     if (e == cudaSuccess && smem > 48 * 1024 && smem > most) {
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e == cudaSuccess) most = smem;
     }
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f.per_sm, kern, threads, smem);
     if (e != cudaSuccess) return cuda_fail(e, what);
-    it = fits.emplace(key, f).first;
+    it = t.fits.emplace(key, f).first;
   }
   *sms = it->second.sms;
   *per_sm = it->second.per_sm;

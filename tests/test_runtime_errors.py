@@ -55,3 +55,15 @@ assert fake.cudaGetLastError() == 0
 print("done")
 """)
     assert "done" in out
+
+
+def test_launch_tables_outlive_the_static_destructors(run):
+    """A server's thread may still launch when the process ends without closing it: the table of
+    kernels' sizes is not destroyed before it (freed memory is overwritten, so a look-up in a
+    destroyed table shows)."""
+    out = run("""
+import sys
+fit = C.cast(lib._ZN2bk10kernel_fitEPKvimPiS2_PKc, C.c_void_p)
+assert fake.fake_fit_at_exit(fit) == 0
+""", GLIBC_TUNABLES="glibc.malloc.tcache_count=0:glibc.malloc.perturb=165")
+    assert "fit after exit: ok" in out
