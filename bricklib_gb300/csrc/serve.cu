@@ -463,6 +463,30 @@ static void serve_loop(bk_server *S) {
   S->cv_done.notify_all();
 }
 
+// A server's streams, events and staging, as many as were made, and the server itself.
+static void release(bk_server *S) {
+  auto stream = [](cudaStream_t s) {
+    if (s) cudaStreamDestroy(s);
+  };
+  auto event = [](cudaEvent_t e) {
+    if (e) cudaEventDestroy(e);
+  };
+  for (int l = 0; l < bk_server::NLANE; ++l) {
+    stream(S->lanes[l]);
+    event(S->join[l]);
+    for (int t = 0; t < bk_server::NTICK; ++t) event(S->tick_ev[t][l]);
+  }
+  event(S->fork);
+  for (size_t r = 0; r < S->ring.size(); ++r) {
+    if (S->ring[r]) cudaFreeHost(S->ring[r]);
+    event(S->ring_ev[r]);
+  }
+  stream(S->s_tick);
+  stream(S->s_admit);
+  stream(S->s_retire);
+  delete S;
+}
+
 }  // namespace bk
 
 extern "C" {
@@ -503,12 +527,12 @@ int bk_server_create(bk_server **out, size_t hbm_budget, const bk_layout *lay, i
   S->ring_ev.assign(K, nullptr);
   for (int r = 0; r < K && e == cudaSuccess; ++r) e = cudaEventCreateWithFlags(&S->ring_ev[r], cudaEventDisableTiming);
   if (e != cudaSuccess) {
-    delete S;
+    release(S);
     return cuda_fail(e, "bk_server_create");
   }
   S->err = device_error_word();
   if (!S->err) {
-    delete S;
+    release(S);
     return fail(BK_ERR_CUDA, "device error word unavailable");
   }
   S->th = std::thread(serve_loop, S);
@@ -629,23 +653,10 @@ int bk_server_destroy(bk_server *S) {
     if (j.grid) cudaFree(j.grid);
     if (j.ready) cudaEventDestroy(j.ready);
   }
-  for (int l = 0; l < bk_server::NLANE; ++l) {
-    cudaStreamDestroy(S->lanes[l]);
-    cudaEventDestroy(S->join[l]);
-    for (int t = 0; t < bk_server::NTICK; ++t) cudaEventDestroy(S->tick_ev[t][l]);
-  }
-  cudaEventDestroy(S->fork);
   if (S->d_doms) cudaFree(S->d_doms);
   if (S->d_work) cudaFree(S->d_work);
   if (S->d_rows) cudaFree(S->d_rows);
-  for (size_t r = 0; r < S->ring.size(); ++r) {
-    if (S->ring[r]) cudaFreeHost(S->ring[r]);
-    if (S->ring_ev[r]) cudaEventDestroy(S->ring_ev[r]);
-  }
-  cudaStreamDestroy(S->s_tick);
-  cudaStreamDestroy(S->s_admit);
-  cudaStreamDestroy(S->s_retire);
-  delete S;
+  release(S);
   return BK_OK;
 }
 

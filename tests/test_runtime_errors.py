@@ -67,3 +67,24 @@ fit = C.cast(lib._ZN2bk10kernel_fitEPKvimPiS2_PKc, C.c_void_p)
 assert fake.fake_fit_at_exit(fit) == 0
 """, GLIBC_TUNABLES="glibc.malloc.tcache_count=0:glibc.malloc.perturb=165")
     assert "fit after exit: ok" in out
+
+
+def test_a_server_that_cannot_be_created_holds_nothing(run):
+    """Whichever of its streams and events cannot be made, and where the device has no error word,
+    bk_server_create gives back what it had made by then."""
+    out = run("""
+create = lambda: lib.bk_server_create(C.byref(C.c_void_p()), C.c_size_t(1 << 30), C.byref(lay), 4)
+fake.fake_fail(0, 0, 1)
+assert create() != 0 and fake.fake_live() == 0, fake.fake_live()
+made = 0
+for n in range(1, 1000):
+    fake.fake_fail(n, 0, 1)  # the n-th stream or event; after the last one the error word
+    assert create() != 0, n
+    assert fake.fake_live() == 0, (n, fake.fake_live())
+    if _abi.lib().bk_last_error().decode().startswith("device error word"):
+        break
+    made = n
+assert made >= 20, made
+print("done")
+""")
+    assert "done" in out
