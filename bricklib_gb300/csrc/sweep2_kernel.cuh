@@ -1369,38 +1369,70 @@ __device__ __forceinline__ void sweep2_brick(const T *rt, T *out_brick, int lt, 
   }
 }
 
-// One (j, i) column of a brick under the 125-point cube with one coefficient per sorted distance, in
-// FP64 on pair sums (58.5 operations per point), for the bricks not computed in fixed point.
+// A brick of the 125-point cube that is not computed in fixed point, in FP64 by one warp, a column
+// pair (j, i0), (j, i0 + 1) per lane (the FP64 pipe, 2 operations per clock and SM, is busy with the six
+// CTAs' one warp each).  Plane by plane the rows j -+ b are added (V, shared by both columns), then the
+// class sums of the plane, then W_a = the sum over the classes of their coefficients at distance a
+// along k, of which each goes to the output planes a below and above: 49 operations per point,
+// no value of one plane kept but four partial outputs per column.  256^3, every brick refused: 1617 us,
+// 1801 for a column per thread on pair sums along k (58.5), 1795 for a column per thread as here (55).
+// (The class sums streamed from brick to brick, 37 operations, take 1166 beside the sums in fixed
+// point, but their registers and code slow those down by 7 %.)
 template <typename C>
-__device__ __forceinline__ void sym_cube_column_f64(const double *rt, double *ob, const int lt, const Taps &tp) {
+__device__ __forceinline__ void sym_cube_planes_f64(const double *rt, double *ob, const int lane, const Taps &tp) {
   constexpr int R = 2, SK = C::SK, SJ = C::EI;
   const F64Ops f = F64Ops::load(tp);
-  const double *col = rt + ((lt >> 3) + R) * SJ + (lt & 7) + C::RP;
-  double acc[8];
+  const double *c = rt + ((lane >> 2) + R) * SJ + 2 * (lane & 3) + C::RP;
+  double *o = ob + 2 * lane;
+  double part[2][4];  // [column]: output planes kk - 4 .. kk - 1 as far as tile planes below kk go
+#pragma unroll
+  for (int q = 0; q < 4; ++q) part[0][q] = part[1][q] = 0.0;
 #pragma unroll 1
-  for (int cls = 0; cls < 6; ++cls) {  // (b, a) = (0,0) (0,1) (1,1) (0,2) (1,2) (2,2)
-    const int a = cls < 1 ? 0 : cls < 3 ? 1 : 2, b = cls == 2 || cls == 4 ? 1 : cls == 5 ? 2 : 0;
-    const double c0 = f64_coef(tp, sym_index(0, b, a, R)), c1 = f64_coef(tp, sym_index(1, b, a, R)),
-                 c2 = f64_coef(tp, sym_index(2, b, a, R));
-    double q[12];
+  for (int kk = 0; kk < 12; ++kk, c += SK) {
+    double V[R + 1][6];  // columns i0 - 2 .. i0 + 3
 #pragma unroll
-    for (int kk = 0; kk < 12; ++kk) {
-      const double *c = col + kk * SK;
-      auto four = [&](int x, int y) {  // rows -+x, columns -+y, each value once
-        const double lo = y ? f.add(c[-x * SJ - y], c[-x * SJ + y]) : c[-x * SJ];
-        if (x == 0) return lo;
-        return f.add(lo, y ? f.add(c[x * SJ - y], c[x * SJ + y]) : c[x * SJ]);
+    for (int m = 0; m < 3; ++m) {
+      const double2 x = ld_pair(c + 2 * m - 2);
+      V[0][2 * m] = x.x;
+      V[0][2 * m + 1] = x.y;
+#pragma unroll
+      for (int b = 1; b <= R; ++b) {
+        const double2 lo = ld_pair(c - b * SJ + 2 * m - 2), hi = ld_pair(c + b * SJ + 2 * m - 2);
+        V[b][2 * m] = f.add(lo.x, hi.x);
+        V[b][2 * m + 1] = f.add(lo.y, hi.y);
+      }
+    }
+    double y[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = 2 + h;
+      auto two = [&](int b, int a) { return f.add(V[b][m - a], V[b][m + a]); };
+      // (b, a) = (0,0) (0,1) (1,1) (0,2) (1,2) (2,2), both orders
+      const double q[6] = {V[0][m], f.add(two(0, 1), V[1][m]), two(1, 1), f.add(two(0, 2), V[2][m]),
+                           f.add(two(1, 2), two(2, 1)), two(2, 2)};
+      auto weighted = [&](int d) {
+        double w = f.mul(f64_coef(tp, sym_index(d, 0, 0, R)), q[0]);
+        w = fma(f64_coef(tp, sym_index(d, 0, 1, R)), q[1], w);
+        w = fma(f64_coef(tp, sym_index(d, 1, 1, R)), q[2], w);
+        w = fma(f64_coef(tp, sym_index(d, 0, 2, R)), q[3], w);
+        w = fma(f64_coef(tp, sym_index(d, 1, 2, R)), q[4], w);
+        return fma(f64_coef(tp, sym_index(d, 2, 2, R)), q[5], w);
       };
-      q[kk] = a == b ? four(b, a) : f.add(four(b, a), four(a, b));
+      const double w2 = weighted(2);
+      y[h] = f.add(part[h][0], w2);  // output plane kk - 4 is complete
+      part[h][0] = part[h][1];
+      part[h][1] = part[h][2];
+      part[h][2] = part[h][3];
+      part[h][3] = w2;
+      if (kk > 0 && kk < 11) {
+        const double w1 = weighted(1);
+        part[h][0] = f.add(part[h][0], w1);
+        part[h][2] = f.add(part[h][2], w1);
+      }
+      if (kk > 1 && kk < 10) part[h][1] = f.add(part[h][1], weighted(0));
     }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const double v = cls ? fma(c0, q[k + 2], acc[k]) : f.mul(c0, q[k + 2]);
-      acc[k] = fma(c2, f.add(q[k], q[k + 4]), fma(c1, f.add(q[k + 1], q[k + 3]), v));
-    }
+    if (kk >= 4) st_pair(o + (kk - 4) * 64, make_double2(y[0], y[1]));
   }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) store_stream(ob + k * 64 + lt, acc[k]);
 }
 
 // Whether one of this thread's rows of a cube's tile holds a value other than zero (64 threads, one brick).
@@ -1784,9 +1816,9 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
           // a cube on zeros (256^3 zeros, us, in FP64 / so: 27-point 755 / 127, 125-point 1798 / 196)
 #pragma unroll
           for (int k = 0; k < 8; ++k) store_stream(reinterpret_cast<double *>(ob) + k * 64 + lt, 0.0);
-        } else if constexpr (C::FX125)
-          sym_cube_column_f64<C>(tile, reinterpret_cast<double *>(ob), lt, tp);
-        else
+        } else if constexpr (C::FX125) {
+          if (lt < 32) sym_cube_planes_f64<C>(tile, reinterpret_cast<double *>(ob), lt, tp);
+        } else
           sweep2_brick<T, BK, BJ, BI, R, FAM, ACCM_NATIVE>(rt, ob, lt, tp, cs);
       } else
         sweep2_brick<T, BK, BJ, BI, R, FAM, ACC>(rt, ob, lt, tp, cs);

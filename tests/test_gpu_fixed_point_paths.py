@@ -9,6 +9,7 @@ import pytest
 from bricklib_gb300 import bricks as B, stencils
 from bricklib_gb300._abi import BK_ACC_NATIVE, BK_F64
 from bricklib_gb300.domain import GridDomain
+from oracle import oracle
 from test_gpu_fixed_point import stencil
 from test_gpu_sweep import _sweep_with
 
@@ -65,6 +66,68 @@ def test_refused_star_bricks_are_the_fp64_chain(name, monkeypatch):
         for t in order:
             v = fma(coeff[t], float(arr[tuple(o[a] + p[a] + t[a] for a in range(3))]), v)
         assert out[tuple(p)] == v, (p, out[tuple(p)], v)
+
+
+def plane_sum(coeff, x):
+    """The 125-point cube at one point as a refused brick sums it, x[5][5][5] its values: plane by
+    plane rows added pairwise, the six class sums of the plane, their weighted sum for the plane's
+    distance along k; the planes' sums added from the lowest to the highest."""
+    total = None
+    for k in range(5):
+        V = [x[k, 2], x[k, 1] + x[k, 3], x[k, 0] + x[k, 4]]
+
+        def two(b, a):
+            return V[b][2 - a] + V[b][2 + a]
+
+        q = [V[0][2], two(0, 1) + V[1][2], two(1, 1), two(0, 2) + V[2][2], two(1, 2) + two(2, 1), two(2, 2)]
+        d, w = abs(k - 2), 0.0
+        for c, v in zip([(0, 0), (0, 1), (1, 1), (0, 2), (1, 2), (2, 2)], q):
+            w = fma(coeff[(d,) + c], float(v), w)
+        total = w if total is None else total + w
+    return total
+
+
+@pytest.mark.parametrize("part", [1.0, 0.5])
+def test_refused_cube125_bricks_are_summed_in_fp64(part, monkeypatch):
+    """The 125-point cube on values that refuse every brick, or about half of them in stretches of
+    one to three, with bricks of zeros between: a refused brick's bits are those of the FP64 sums
+    plane by plane, and no brick's depend on what the list has around it."""
+    st = stencil("cube125")
+    dom = domain((24, 32, 128))
+    rng = np.random.default_rng(5)
+    arr = wide(dom.adims)
+    if part < 1:
+        plain = stencils.uniform(78, arr.size).reshape(arr.shape)
+        calm = rng.random([m // 8 for m in arr.shape]) >= 0.02
+        arr = np.where(np.repeat(np.repeat(np.repeat(calm, 8, 0), 8, 1), 8, 2), plain, arr)
+    arr[dom.org[0]:, :, dom.org[2] + 40:dom.org[2] + 60] = 0.0  # bricks of zeros
+    dom.set_field(0, arr)
+    dom.upload()
+    it = np.asarray(dom.interior, dtype=np.uint32)
+    cuts = np.cumsum(rng.integers(1, 6, size=len(it)))
+    pieces = np.split(it, cuts[cuts < len(it)])
+    lists = {"grid": it, "shuffled": rng.permutation(it),
+             "pieces": np.concatenate([pieces[p] for p in rng.permutation(len(pieces))]),
+             "repeats": np.repeat(it, rng.integers(1, 3, size=len(it)))}
+    full = None
+    for key, lst in lists.items():
+        got = _sweep_with(None, monkeypatch, dom, st, BK_ACC_NATIVE, B.BrickList(np.ascontiguousarray(lst)))
+        full = got if full is None else full
+        np.testing.assert_array_equal(got.view(np.uint8), full.view(np.uint8), err_msg=key)
+    out = interior(dom, full)
+    coeff = {t: float(c) for t, c in zip([tuple(t) for t in st.taps], st.coeff)}
+    o, same = dom.org, 0
+    pts = points(dom, 600)
+    for p in pts:
+        x = arr[tuple(slice(o[a] + p[a] - 2, o[a] + p[a] + 3) for a in range(3))]
+        same += out[tuple(p)] == plane_sum(coeff, x)
+    # every point of a refused brick; of the accepted ones only those whose two roundings agree
+    assert same == len(pts) if part == 1 else 0.2 * len(pts) < same < 0.95 * len(pts), same
+    want = np.zeros_like(arr)
+    oracle.array_sweep(arr, want, o, tuple(a + b for a, b in zip(o, dom.n)), st.offsets(), st.coeff)
+    size = np.zeros_like(arr)
+    oracle.array_sweep(np.abs(arr), size, o, tuple(a + b for a, b in zip(o, dom.n)), st.offsets(), np.abs(st.coeff))
+    assert (np.abs(out - dom.interior_view(want)) <= 3 * 125 * 2.0 ** -53 * dom.interior_view(size)).all()
 
 
 @pytest.mark.parametrize("name", ["star7", "heat7", "star13", "star25", "cube27", "cube125"])
