@@ -253,7 +253,7 @@ int batch_dispatch(const BatchStencil &bs, const BatchDomain *doms, unsigned ndo
         if (p.sym && p.fam == FAM_CUBE && p.r == 2) return launch_sweep2<T, 8, 8, 8, 2, FAM_CUBESYM, ACC, true, true>(a, tp, s, grid_cap);
       }
       if constexpr (sizeof(T) <= 4 && ACC == ACCM_NATIVE)  // ... and the radius-1 cube without the symmetry
-        if (!p.sym && p.fam == FAM_CUBE && p.r == 1) return launch_sweep2<T, 8, 8, 8, 1, FAM_CUBE, ACC, true, true>(a, tp, s, grid_cap);
+        if (!p.sym && p.fam == FAM_CUBE && p.r == 1) return launch_cube27<T, true>(a, tp, s, grid_cap);
       if constexpr (ACC == ACCM_NATIVE) {  // mirror-symmetric cubes: the pair-sum variant
         if (p.symij && p.fam == FAM_CUBE && p.r == 1) return launch_sweep2<T, 8, 8, 8, 1, FAM_CUBESYM_IJ, ACC, true>(a, tp, s, grid_cap);
         if (p.symij && p.fam == FAM_CUBE && p.r == 2) return launch_sweep2<T, 8, 8, 8, 2, FAM_CUBESYM_IJ, ACC, true>(a, tp, s, grid_cap);

@@ -231,9 +231,9 @@ struct Sweep2Cfg {
   static constexpr int EPT = DEFER ? EPT_MID + EPT_SIDE : (NV + TPB - 1) / TPB;  // plan entries per thread
   // copies whose source addresses are read together.  GB300 at 512^3, us, one / two / three / four:
   // FP32 cube125 460 / 454 / 455 / 460, FP64 cube125 2199 / 2161 / 2159 / 2154, BF16 cube125 376 / 378 /
-  // 381 / 384; the other 4- and 2-byte kernels, whose warps are many, one: FP32 cube27 425 / 447, BF16
-  // 304 / 312
-  static constexpr int ISSUE = IST || ES == 8 ? 2 : 1;
+  // 381 / 384; the column pairs of the radius-1 cube on the same storage, which run short lists
+  // (launch_cube27), two (8 bricks, FP32 3.14 / 3.00, BF16 3.31 / 3.20); the other 4- and 2-byte kernels one
+  static constexpr int ISSUE = IST || ES == 8 || (PAIR && FAM == FAM_CUBE) ? 2 : 1;
   // float-float converts each raw FP64 tile into float pairs in place (same 8 bytes)
   static constexpr int FTILE_BYTES = 0;
   // bricks per CTA: as many as fit 128 threads and a ~100 KB shared-memory budget
@@ -412,26 +412,28 @@ __device__ __forceinline__ void cube_pair_columns(const T *rt, T *ob, const int 
     }
   };
   if constexpr (FAM == FAM_CUBE) {
+    static_assert(R == 1, "radius-1 cube");
 #pragma unroll
     for (int kk = 0; kk < NK; ++kk) {
       load_plane(kk);
       if (kk >= 2 * R) {
         const int k = kk - 2 * R;
-        AT acc[2];
+        AT w[3][2];  // the sum per tap offset along i, then theirs: the order of cube_istream4, the same bits
 #pragma unroll
-        for (int dj = -R; dj <= R; ++dj)
+        for (int di = -R; di <= R; ++di)
 #pragma unroll
-          for (int di = -R; di <= R; ++di)
+          for (int dk = -R; dk <= R; ++dk)
 #pragma unroll
-            for (int dk = -R; dk <= R; ++dk) {
+            for (int dj = -R; dj <= R; ++dj) {
               const int t = ((dk + R) * (2 * R + 1) + (dj + R)) * (2 * R + 1) + (di + R);
               const AT c = coef<AT>(tp, t);
 #pragma unroll
               for (int o = 0; o < 2; ++o) {
                 const AT v = x[k + R + dk][dj + R][R + o + di];
-                acc[o] = (dj == -R && di == -R && dk == -R) ? c * v : fma(c, v, acc[o]);
+                w[di + R][o] = (dj == -R && dk == -R) ? c * v : fma(c, v, w[di + R][o]);
               }
             }
+        const AT acc[2] = {(w[0][0] + w[1][0]) + w[2][0], (w[0][1] + w[1][1]) + w[2][1]};
         st_pair(ob + k * PK, pair_of(acc[0], acc[1]));
       }
     }
@@ -1862,6 +1864,27 @@ int launch_sweep2(const SweepArgs &a, const Taps &tp, cudaStream_t s, int grid_c
   }
   if (e != cudaSuccess) return cuda_fail(e, "sweep2 kernel launch");
   return BK_OK;
+}
+
+// The radius-1 cube without mirror symmetry on 4- and 2-byte storage: streamed (cube_istream4) where every
+// resident CTA gets several bricks, on column pairs where not, which give the same bits: with a brick
+// or two per CTA there is no run to gain from, and the stream's edge columns and its longer start are
+// lost.  Lists in grid order, us per sweep in a captured graph, stream / pairs: FP32 8 bricks 3.6 / 3.0, 1728
+// 7.0 / 6.4, 4096 11.1 / 10.2, 6156 13.4 / 13.6, 13824 20.5 / 25.1; BF16 1728 6.2 / 5.4, 2744 7.6 / 6.7, 4096
+// 9.2 / 9.5, 13824 17.2 / 21.2 (2128 and 2432 CTAs).  The line: 2.5 bricks per CTA, BF16 1.5.
+template <typename T, bool BATCH>
+int launch_cube27(const SweepArgs &a, const Taps &tp, cudaStream_t s, int grid_cap = 0) {
+  typedef Sweep2Cfg<T, 8, 8, 8, 1, FAM_CUBE, ACCM_NATIVE, true> C;
+  static_assert(sizeof(T) <= 4, "FP32 / BF16 storage");
+  auto kern = sweep2_kernel<T, 8, 8, 8, 1, FAM_CUBE, ACCM_NATIVE, BATCH, true>;
+  int sms = 0, per_sm = 0;
+  const int st = kernel_fit(reinterpret_cast<const void *>(kern), C::NT, C::SMEM, &sms, &per_sm, "sweep2 launch setup");
+  if (st) return st;
+  long long ctas = (long long)sms * per_sm;
+  if (grid_cap > 0 && ctas > grid_cap) ctas = grid_cap;
+  if (2 * (long long)a.nlist < (sizeof(T) == 4 ? 5 : 3) * ctas)
+    return launch_sweep2<T, 8, 8, 8, 1, FAM_CUBE, ACCM_NATIVE, BATCH>(a, tp, s, grid_cap);
+  return launch_sweep2<T, 8, 8, 8, 1, FAM_CUBE, ACCM_NATIVE, BATCH, true>(a, tp, s, grid_cap);
 }
 
 // Tile geometry the host needs for generic-family tap offsets.

@@ -46,9 +46,8 @@ int sweep_dispatch_f32(const SweepPlan &p, const SweepArgs &a, Taps &tp, cudaStr
         if (p.r == 1) return launch_sweep2<float, 8, 8, 8, 1, FAM_CUBESYM, ACCM_COMP, false, true>(a, tp, s);
         if (p.r == 2) return launch_sweep2<float, 8, 8, 8, 2, FAM_CUBESYM, ACCM_COMP, false, true>(a, tp, s);
       }
-      // the radius-1 cube without it: three weighted column sums streamed the same way
-      if (!p.sym && p.fam == FAM_CUBE && p.istream)
-        return launch_sweep2<float, 8, 8, 8, 1, FAM_CUBE, ACCM_NATIVE, false, true>(a, tp, s);
+      // the radius-1 cube without it: three weighted column sums streamed the same way, on long lists
+      if (!p.sym && p.fam == FAM_CUBE && p.istream) return launch_cube27<float, false>(a, tp, s);
       // ... one brick at a time on column pairs (BK_SWEEP_ISTREAM=0)
       if (p.sym && p.fam == FAM_CUBE && p.acc == ACCM_NATIVE) {
         if (p.symij && p.r == 1) return launch_sweep2<float, 8, 8, 8, 1, FAM_CUBESYM_IJ, ACCM_NATIVE>(a, tp, s);
