@@ -8,10 +8,14 @@
 //              and the tick stream waits on that before the job's first step;
 //   ticks      every active job advances one step per tick: one persistent sweep launch per
 //              (storage type, stencil) group over a work list of the group's jobs' bricks.  The
-//              groups share no data, so each runs its ticks on a stream of its own (lanes), and a
-//              group of few bricks does not leave the GPU idle while it runs; the lanes meet
-//              only where the work lists change.  Jobs join and leave between ticks, so work of
-//              jobs that arrived at different times overlaps;
+//              groups share no data.  Those on FP64 storage, whose sweeps are long against a
+//              hand-over between streams, run their ticks each on a stream of its own (lanes),
+//              so that a group of few bricks does not leave the GPU idle while it runs; those on
+//              FP32 storage follow each other on the tick stream; the lanes meet where the work
+//              lists change.  24 small FP32 jobs (to 48^3, 60 steps), ms: a lane each 2.95, on the
+//              tick stream 2.65 (one stream for everything 2.54 to 2.66, on the same boxes); 24 jobs
+//              of both types to 128^3: 4.9 either way (one stream 8.2).  Jobs join and leave between
+//              ticks, so work of jobs that arrived at different times overlaps;
 //   retirement after its last step a job's newest field is gathered into an array and
 //              copied to the client's output on a retire stream; a host callback on that
 //              stream stamps the completion time, releases its budget and wakes waiters.
@@ -139,11 +143,17 @@ struct bk_server {
   BatchDomain *d_doms = nullptr;
   uint2 *d_work = nullptr;
   JobRow *d_rows = nullptr;
-  std::vector<std::pair<int, std::pair<unsigned, unsigned>>> work_seg;  // group -> (offset, count)
+  struct Segment {  // a group's part of the work list, and the lane it runs on
+    int group;
+    unsigned offset, count;
+    int lane;
+  };
+  std::vector<Segment> work_seg;
   unsigned ndom = 0;
   int parity = 0;
-  // lanes: group q of the tick program runs on lane q mod NLANE.  fork: the program's tables are on
-  // the device; tick_ev[t mod NTICK][lane]: the lane is through tick t (bits of tick_used: lanes in use)
+  // lane 0 is the tick stream.  fork: the program's tables are on the device; join: the lane is through
+  // its ticks of the program before; tick_ev[t mod NTICK][lane]: the lane is through tick t (bits of
+  // tick_used: lanes in use)
   static constexpr int NLANE = 8, NTICK = 4;
   cudaStream_t lanes[NLANE] = {};
   cudaEvent_t fork = nullptr, join[NLANE] = {}, tick_ev[NTICK][NLANE] = {};
@@ -244,8 +254,8 @@ static int admit(bk_server *S, const std::shared_ptr<Job> &j) {
 
 // Lane of a group in the current tick program.
 static int lane_of(const bk_server *S, int group) {
-  for (size_t q = 0; q < S->work_seg.size(); ++q)
-    if (S->work_seg[q].first == group) return (int)(q % bk_server::NLANE);
+  for (const auto &seg : S->work_seg)
+    if (seg.group == group) return seg.lane;
   return 0;
 }
 
@@ -304,7 +314,7 @@ static unsigned char *ring_slot(bk_server *S, size_t bytes, int *slot) {
 // ticks of the program before (which read the tables freed here), before their next ones
 static int rebuild(bk_server *S) {
   cudaStream_t s = S->s_tick;
-  for (int l = 0; l < bk_server::NLANE; ++l)
+  for (int l = 1; l < bk_server::NLANE; ++l)
     if ((S->lanes_used >> l) & 1u) {
       BK_CUDA(cudaEventRecord(S->join[l], S->lanes[l]));
       BK_CUDA(cudaStreamWaitEvent(s, S->join[l], 0));
@@ -319,6 +329,8 @@ static int rebuild(bk_server *S) {
   std::vector<JobRow> rows(n);
   S->work_seg.clear();
   unsigned long long woff = 0;
+  int next = 0;
+  unsigned wanted = 0;
   for (unsigned d = 0; d < n; ++d) {
     const Job &j = *order[d];
     const size_t es = dtype_size(j.dtype);
@@ -328,9 +340,12 @@ static int rebuild(bk_server *S) {
                           (unsigned long long)2 * S->L.size() * es, j.nbricks};
     const unsigned long long nint = (unsigned long long)(j.g[0] - 2) * (j.g[1] - 2) * (j.g[2] - 2);
     rows[d] = JobRow{d, j.g[0], j.g[1], j.g[2], woff};
-    if (S->work_seg.empty() || S->work_seg.back().first != j.group)
-      S->work_seg.push_back({j.group, {(unsigned)woff, 0}});
-    S->work_seg.back().second.second += (unsigned)nint;
+    if (S->work_seg.empty() || S->work_seg.back().group != j.group) {
+      const int lane = j.dtype == BK_F64 ? 1 + next++ % (bk_server::NLANE - 1) : 0;
+      S->work_seg.push_back({j.group, (unsigned)woff, 0, lane});
+      wanted |= 1u << lane;
+    }
+    S->work_seg.back().count += (unsigned)nint;
     woff += nint;
   }
   // new device buffers (stream ordered); the previous ones are freed after the ticks using them
@@ -356,8 +371,9 @@ static int rebuild(bk_server *S) {
   BK_CUDA(cudaEventRecord(S->ring_ev[slot], s));
   expand_work_kernel<<<n, 256, 0, s>>>(S->d_rows, n, S->d_work);
   BK_CUDA(cudaGetLastError());
-  BK_CUDA(cudaEventRecord(S->fork, s));
-  for (int l = 0; l < bk_server::NLANE; ++l) BK_CUDA(cudaStreamWaitEvent(S->lanes[l], S->fork, 0));
+  if (wanted & ~1u) BK_CUDA(cudaEventRecord(S->fork, s));
+  for (int l = 1; l < bk_server::NLANE; ++l)
+    if ((wanted >> l) & 1u) BK_CUDA(cudaStreamWaitEvent(S->lanes[l], S->fork, 0));
   S->active = order;
   return BK_OK;
 }
@@ -365,15 +381,13 @@ static int rebuild(bk_server *S) {
 static int tick(bk_server *S) {
   const int slot = (int)(S->ticks % bk_server::NTICK);
   unsigned used = 0;
-  int q = 0;
-  for (auto &ws : S->work_seg) {
-    const Group &g = S->groups[ws.first];
-    const int l = q++ % bk_server::NLANE;
+  for (const auto &seg : S->work_seg) {
+    const Group &g = S->groups[seg.group];
     // job storages come from cudaMallocAsync and hold two whole-brick fields: aligned
-    int st = batch_launch_sweep(g.bs, g.dtype, S->d_doms, S->ndom, S->d_work + ws.second.first, ws.second.second,
-                                S->parity, S->L, S->err, 0, true, S->lanes[l]);
+    int st = batch_launch_sweep(g.bs, g.dtype, S->d_doms, S->ndom, S->d_work + seg.offset, seg.count,
+                                S->parity, S->L, S->err, 0, true, S->lanes[seg.lane]);
     if (st) return st;
-    used |= 1u << l;
+    used |= 1u << seg.lane;
   }
   for (int l = 0; l < bk_server::NLANE; ++l)
     if ((used >> l) & 1u) BK_CUDA(cudaEventRecord(S->tick_ev[slot][l], S->lanes[l]));
@@ -472,7 +486,7 @@ static void release(bk_server *S) {
     if (e) cudaEventDestroy(e);
   };
   for (int l = 0; l < bk_server::NLANE; ++l) {
-    stream(S->lanes[l]);
+    if (l) stream(S->lanes[l]);
     event(S->join[l]);
     for (int t = 0; t < bk_server::NTICK; ++t) event(S->tick_ev[t][l]);
   }
@@ -508,8 +522,9 @@ int bk_server_create(bk_server **out, size_t hbm_budget, const bk_layout *lay, i
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&S->s_retire, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&S->fork, cudaEventDisableTiming);
   for (int l = 0; l < bk_server::NLANE && e == cudaSuccess; ++l) {
-    e = cudaStreamCreateWithFlags(&S->lanes[l], cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&S->join[l], cudaEventDisableTiming);
+    if (l == 0) S->lanes[0] = S->s_tick;
+    else e = cudaStreamCreateWithFlags(&S->lanes[l], cudaStreamNonBlocking);
+    if (e == cudaSuccess && l) e = cudaEventCreateWithFlags(&S->join[l], cudaEventDisableTiming);
     for (int t = 0; t < bk_server::NTICK && e == cudaSuccess; ++t)
       e = cudaEventCreateWithFlags(&S->tick_ev[t][l], cudaEventDisableTiming);
   }
