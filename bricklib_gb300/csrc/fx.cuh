@@ -47,6 +47,7 @@ struct FxTab {
   int w[8];                      // weights of the checked terms, by neighbour: 1 i, 2 j, 4 k
   int elo, ehi;                  // range of E
   int q;                         // C = c 2^q
+  int zeros;                     // sums of +0 are +0 (they are -0 where all coefficients are negative)
 };
 
 bool fx_table(const double *c, int n, const int (*near)[9], int masks, int slots, const int *first, const int *count,
@@ -595,14 +596,14 @@ __device__ __forceinline__ bool fx_prepare(const Share &sh, const double *from, 
   if (stopped || !on) return false;
   const FxScan s = fx_gather(slot);
   E = (int)(s.top >> 20);
-  // a star on zeros, or numbers below 2^-1042: where all are zero, so are the sums, on any scale (256^3
+  // a star on zeros, or numbers below 2^-1042: where all are +0, so are the sums, on any scale (256^3
   // zeros, us, in FP64 / so: 7-point 197 / 89, 13-point 359 / 104, 25-point 689 / 162; the cubes
   // write their zeros themselves, sweep2_kernel)
-  if (Share::STAR && s.top == 0) {
+  if (Share::STAR && s.top == 0 && tab.zeros) {
     if constexpr (!Share::HOLD) sh.load(from, v);
     bool some = false;
 #pragma unroll
-    for (int q = 0; q < Share::NV; ++q) some = some || __double2loint(v[q]) != 0;
+    for (int q = 0; q < Share::NV; ++q) some = some || __double_as_longlong(v[q]) != 0;
     if (fx_bar_or(brick, some)) return false;
     E = tab.elo;
   } else if (!fx_ok(tab, s)) {

@@ -42,9 +42,11 @@ bool fx_table(const double *c, int n, const int (*near)[9], int masks, int slots
   t->on = 0;
   double sum = 0.0, most = 0.0, heads = 0.0;
   bool exact = true;  // c[k] x exact for every k but the centre
+  t->zeros = 0;
   for (int k = 0; k < n; ++k) {
     sum += fabs(c[k]);
     most = fmax(most, fabs(c[k]));
+    if (!std::signbit(c[k])) t->zeros = 1;
     int e;
     if (k != near[0][0] && c[k] != 0.0) exact = exact && fabs(frexp(c[k], &e)) == 0.5;
   }

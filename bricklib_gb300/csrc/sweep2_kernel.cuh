@@ -1440,14 +1440,14 @@ __device__ __forceinline__ void sym_cube_planes_f64(const double *rt, double *ob
   }
 }
 
-// Whether one of this thread's rows of a cube's tile holds a value other than zero (64 threads, one brick).
+// Whether one of this thread's rows of a cube's tile holds a value other than +0 (64 threads, one brick).
 template <typename C, int R>
 __device__ __forceinline__ bool cube_tile_nonzero(const double *rt, const int lt) {
   bool some = false;
 #pragma unroll 1
   for (int r = lt; r < C::EK * C::EJ; r += 64) {
     const double *row = rt + r / C::EJ * C::SK + r % C::EJ * C::EI + C::RP - R;
-    for (int i = 0; i < 8 + 2 * R; ++i) some = some || row[i] != 0.0;
+    for (int i = 0; i < 8 + 2 * R; ++i) some = some || __double_as_longlong(row[i]) != 0;
   }
   return some;
 }
@@ -1824,7 +1824,7 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
         double *tile = reinterpret_cast<double *>(const_cast<T *>(rt));
         if (fx_prepare(share, tile, tile, tp.fx, scan + 2 * NB * cur, slot, E, true, false, stopped, [] {}))
           sweep2_brick_fx<T, R, FAM, ACC>(tile, ob, lt, tp, E);
-        else if (FAM == FAM_CUBE && E == 0 && !fx_bar_or(slot, cube_tile_nonzero<C, R>(tile, lt))) {
+        else if (FAM == FAM_CUBE && E == 0 && tp.fx.zeros && !fx_bar_or(slot, cube_tile_nonzero<C, R>(tile, lt))) {
           // a cube on zeros (256^3 zeros, us, in FP64 / so: 27-point 755 / 127, 125-point 1798 / 196)
 #pragma unroll
           for (int k = 0; k < 8; ++k) store_stream(reinterpret_cast<double *>(ob) + k * 64 + lt, 0.0);

@@ -14,7 +14,7 @@ TAPS = 27
 
 class Table(C.Structure):
     _fields_ = [("on", C.c_int), ("ch", C.c_int * TAPS), ("cl", C.c_int * TAPS), ("w", C.c_int * 8),
-                ("elo", C.c_int), ("ehi", C.c_int), ("q", C.c_int)]
+                ("elo", C.c_int), ("ehi", C.c_int), ("q", C.c_int), ("zeros", C.c_int)]
 
 
 def tap_list(kind, r):
