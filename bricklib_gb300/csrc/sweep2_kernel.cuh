@@ -1462,23 +1462,17 @@ __device__ __forceinline__ void sweep2_brick_fx(const double *rt, double *out_br
     const int j = (lt & 3) | ((lt >> 1) & 4), k = ((lt >> 2) & 1) | ((lt >> 3) & 6);
     const double *c = rt + (k + R) * SK + (j + R) * SJ;
     double *o = out_brick + k * 64 + j * 8;
-    const bool two = (reinterpret_cast<uintptr_t>(o) & 15) == 0;
     fx_cube125_row([&](int dk, int dj, int p) { return ld_pair(c + dk * SK + dj * SJ + 2 * p); },
-                   [&](int p, double y0, double y1) {
-                     if (two) st_pair(o + 2 * p, make_double2(y0, y1));
-                     else {
-                       store_stream(o + 2 * p, y0);
-                       store_stream(o + 2 * p + 1, y1);
-                     }
-                   },
-                   tp.fx, fx_scale<58>(E, tp.fx.q));
+                   [&](int p, double y0, double y1) { st_pair(o + 2 * p, make_double2(y0, y1)); }, tp.fx,
+                   fx_scale<58>(E, tp.fx.q));
     return;
   } else {
   // four planes of a column pair; a quarter warp takes rows two apart, which fall in different banks
   const int q = (lt >> 2) & 7, j = (q & 4) | ((q & 1) << 1) | ((q >> 1) & 1), i = 2 * (lt & 3), k0 = 4 * (lt >> 5);
   const double *c = rt + (k0 + R) * SK + (j + R) * SJ + i + C::RP;
   double *o = out_brick + k0 * 64 + j * 8 + i;
-  const bool two = (reinterpret_cast<uintptr_t>(o) & 15) == 0;  // output bricks may start anywhere
+  // a star's output bricks may start anywhere (cubes come here with pairs that may be stored, plan_sweep)
+  const bool two = FAM == FAM_CUBE || (reinterpret_cast<uintptr_t>(o) & 15) == 0;
   auto put = [&](int k, double y0, double y1) {
     if (two) st_pair(o + k * 64, make_double2(y0, y1));
     else {
