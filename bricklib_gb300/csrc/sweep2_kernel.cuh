@@ -260,10 +260,10 @@ struct Sweep2Cfg {
   // for 14); the compensated stream (two warps per CTA): BK_CS_COMP_MINB
   // the fixed-point cubes: radius 1 five CTAs of two bricks (256^3: 236 us; four 244, three 261),
   // the 125-point one six of one brick (298 us; seven 301 with fewer registers)
-  // the others on 4- and 2-byte storage four: asked for nothing, the compiler holds the stars to 40
+  // the others on 4- and 2-byte storage with CTAs of up to 128 threads four: asked for nothing, the compiler holds the stars to 40
   // registers and their loads stand in line (us in a captured graph, nothing / four / eight: FP32 13-point
   // 32^3 3.34 / 2.77 / 2.76, 96^3 6.61 / 5.80 / 6.00, 224^3 43.7 / 38.4 / 38.9, compensated 25-point 224^3 124 / 83 / 127)
-  static constexpr int MINB = CS4 ? (ACC == ACCM_NATIVE ? (R > 1 ? 11 : DEFER && ES == 4 ? 14 : 16) : BK_CS_COMP_MINB) : FX125 ? 6 : FX && FAM == FAM_CUBE ? 5 : ES <= 4 ? 4 : 0;
+  static constexpr int MINB = CS4 ? (ACC == ACCM_NATIVE ? (R > 1 ? 11 : DEFER && ES == 4 ? 14 : 16) : BK_CS_COMP_MINB) : FX125 ? 6 : FX && FAM == FAM_CUBE ? 5 : ES <= 4 && NT <= 128 ? 4 : 0;
 };
 
 // Tile coordinates (kk, jj, ii) of plan vector g for the star / cube neighbourhood.
@@ -1617,7 +1617,9 @@ sweep2_kernel(const SweepArgs a, const Taps tp) {
   };
   auto store_adj = [&](int ns, const Fetched &f) {
     Staged &nb = nbrs[ns * NB + slot];
-    if (!STREAM && !f.listed) {  // no brick: its addresses are not read (streams: 512^3 FP32 cube27 281 us, 293 with this)
+    // no brick: its addresses are not read (streams and FP64 keep their registers better without this
+    // branch: 512^3 FP32 cube27 281 us, 293 with it, FP64 4x4x4 bricks 3 % slower)
+    if (!STREAM && C::ES <= 4 && !f.listed) {
       if (lt == 13) {
         nb.active = 0;
         if (f.alive) atomicOr(a.err, FLAG_BOUNDS);

@@ -50,8 +50,11 @@ typedef enum bk_dtype { BK_F64 = 0, BK_F32 = 1, BK_BF16 = 2 } bk_dtype;
 /* Arithmetic of a sweep.
  * BK_ACC_NATIVE      accumulate in the storage type (FP32 for BF16 storage); FP64 stars and cubes on
  *                    row-major 8x8x8 bricks (and 4-D radius-1 stars) sum bricks whose values allow it
- *                    in 64-bit fixed point, the sum rounded once: closer to the exact sum than the
- *                    FP64 chain, zero sums are +0; the other bricks in FP64
+ *                    in 64-bit fixed point, the sum rounded once, the other bricks in FP64.  The
+ *                    error of n terms is at most n 2^-53 of the largest term, the bound of the FP64
+ *                    chain, and the rounding of the result (on uniform values a few times smaller
+ *                    than the chain's error); a point's last bits depend on the values around it in
+ *                    its brick
  * BK_ACC_COMPENSATED FP32/BF16 storage: FP32 accumulation with Neumaier compensation
  * BK_ACC_FLOATFLOAT  FP64 storage: products and sums in float-float (pairs of FP32,
  *                    error-free transforms of Dekker 1971 / Knuth TwoSum), relative
